@@ -207,13 +207,13 @@ int rgs_batch_add(rgs_batch* batch, rgs_plan* plan, const double* unitaries, con
                   void* sample_value, double* sample_logscale, double* sample_logp, int32_t* index);
 int rgs_batch_info(const rgs_batch* batch, int32_t* instances, int64_t* units);
 /* Queues the whole batch on stream.  The first run after rgs_batch_add uploads the work
- * list (synchronous); later runs are two stream operations (a counter reset and one
+ * list (synchronous); later runs are two stream operations (a status reset and one
  * kernel).  check != 0 synchronises and reports a zero-mass branch pair as
  * RGS_ERR_ZERO_NORM. */
 int rgs_batch_run(rgs_batch* batch, int32_t check, void* stream);
 /* Autotuning of the batch's launch: runs it with each launch variant that holds every
- * instance (one 512-thread block per SM with 192 KiB of tables, two 256-thread blocks with
- * 94 KiB, or four 128-thread blocks with 44 KiB) and keeps the fastest; *variant = the
+ * instance (512-thread blocks with 192 KiB of tables, 128-thread blocks with 56 KiB or
+ * with 36 KiB) and keeps the fastest; *variant = the
  * chosen one, ms[3] = milliseconds per run (-1 where a variant does not fit; may be
  * NULL).  Runs the batch (outputs are written); synchronises.  No counterpart in the
  * reference (it has no batch launch). */

@@ -81,10 +81,8 @@ int rgs_batch_add(rgs_batch* batch, rgs_plan* plan, const double* unitaries, con
     if (o && (rc = same_device(batch, o))) return rc;
   const Plan::DeviceCopy* dc = nullptr;
   if ((rc = plan_device_copy(p, batch->dev.device, &dc))) return rc;
-  ResInstance in;
-  in.steps = (const DevStep*)dc->steps;
-  in.tables = (const unsigned long long*)dc->tables;
-  in.verts = (const DevVert*)dc->verts;
+  ResInstance in{};
+  in.steps = (const ResStep*)dc->res;
   in.U = unitaries;
   in.bits = (const unsigned long long*)bits;
   in.out_value = out_value;
@@ -171,10 +169,10 @@ int rgs_batch_run(rgs_batch* batch, int32_t check, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if ((rc = resident_launch(batch->dev, batch->precision, s, nullptr))) return rc;
   if (check) {
-    int h[2] = {0, 0};
-    RGS_CUDA_TRY(cudaMemcpyAsync(h, batch->dev.counter, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    int h = 0;
+    RGS_CUDA_TRY(cudaMemcpyAsync(&h, batch->dev.status, sizeof(int), cudaMemcpyDeviceToHost, s));
     RGS_CUDA_TRY(cudaStreamSynchronize(s));
-    if (h[1]) return fail(RGS_ERR_ZERO_NORM, "a branch pair had zero or non-finite total mass");
+    if (h) return fail(RGS_ERR_ZERO_NORM, "a branch pair had zero or non-finite total mass");
   }
   return RGS_OK;
 }

@@ -362,6 +362,42 @@ void build_pairs(Plan& p) {
   p.tables.insert(p.tables.end(), mb.begin(), mb.end());
 }
 
+// On-chip step records (plans of rank <= kResMaxRank): see ResStep.
+void build_resident(Plan& p) {
+  p.res.clear();
+  if (p.rmax > kResMaxRank) return;
+  for (int j = 0; j < p.n; ++j) {
+    const DevStep& d = p.dev[j];
+    const PlanStep& st = p.steps[j];
+    ResStep r{};
+    r.r_in = d.r_in;
+    r.v = d.v;
+    r.mode = d.mode;
+    r.t = (unsigned)d.t;
+    r.lrows = d.mode == MODE_PAIR ? d.r_out - 1 : d.r_out;
+    auto parity = [&](unsigned long long c) {
+      return (unsigned)(__builtin_popcountll(c & ((1ull << d.r_in) - 1ull) & d.beta) & 1);
+    };
+    for (int i = 0; i < r.lrows; ++i) {
+      // Pair mode: the row index skips the pivot bit of t (deposit_zero).
+      const int pos = (d.mode == MODE_PAIR && i >= d.pi) ? i + 1 : i;
+      const unsigned long long l = (unsigned long long)st.lcols[pos];
+      const unsigned y = (unsigned)((l >> d.r_in) & 1ull);
+      const unsigned out = (1u << pos) ^ ((d.mode == MODE_PAIR && y) ? (unsigned)d.t : 0u);
+      r.col[i] = (unsigned)l | (parity(l) << 15) | (out << 16);
+    }
+    for (int k = 0; k < d.ncombos; ++k) r.combo[k] = (unsigned)d.combos[k] | (parity(d.combos[k]) << 15);
+    if (d.mode == MODE_PAIR)
+      r.code = d.ncombos == 1 ? RC_P1
+                              : (d.ncombos == 2 ? (d.ng0 == 2 ? RC_P2F : RC_P2H) : (d.ng0 == 4 ? RC_P4F : RC_P4H));
+    else
+      r.code = d.ncombos == 1 ? RC_M1 : RC_M2;
+    const u128 f = p.future[j];
+    for (int w = 0; w < 4; ++w) r.fut[w] = (unsigned)(f >> (32 * w));
+    p.res.push_back(r);
+  }
+}
+
 // Builds the device records; fails (without error) when a step is too wide to execute.
 void build_device(Plan& p) {
   p.dev.clear();
@@ -417,6 +453,7 @@ void build_device(Plan& p) {
     for (int k = 0; k < 4; ++k) d.combos[k] = k < d.ncombos ? (unsigned long long)combos[k] : 0ull;
     p.dev.push_back(d);
   }
+  build_resident(p);
   build_pairs(p);
 }
 

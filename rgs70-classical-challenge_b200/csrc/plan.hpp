@@ -58,6 +58,28 @@ struct DevStep {
   int ng0;                       // MODE_PAIR: the first ng0 combos have y bit 0 (the rest y bit 1)
 };
 
+// Step record of the on-chip sweep (resident.cu): 32 words, so that one warp fetches a
+// record with one coalesced 128-byte load.  Everything a row needs follows from one
+// GF(2)-linear word of the row index r, q(r) = XOR of col[i] over the set bits of r:
+//   bits 0..14  L c' of the row's first output (c, and the y bit at r_in)
+//   bit 15      parity(c & beta)
+//   bits 16..   the output row that takes the kappa-0 combos' f(0) terms: c' itself or,
+//               where the row's y bit is 1, its pair partner c' ^ t
+// and combo k shifts bits 0..15 by the constant combo[k].  Ranks up to kResMaxRank.
+constexpr int kResMaxRank = 13;
+enum ResCode : int { RC_P1 = 0, RC_P2H = 1, RC_P2F = 2, RC_P4H = 3, RC_P4F = 4, RC_M1 = 5, RC_M2 = 6 };
+struct ResStep {
+  unsigned col[13];              // word of row-index bit i
+  unsigned combo[4];             // the step's combos (order of DevStep), parity bit at 15
+  unsigned t;                    // pair partner offset (0 in merge / fixed mode)
+  int code;                      // ResCode: mode, number of combos, kappa pattern
+  int r_in, lrows;               // input rank; log2 of the rows (pair mode: of row pairs)
+  int v, mode;                   // vertex; StepMode
+  unsigned fut[4];               // later-neighbour mask (fixed vertices)
+  unsigned pad[5];
+};
+static_assert(sizeof(ResStep) == 128, "one 128-byte record per position");
+
 // Two consecutive free positions A = j and B = j + 1 run as one pass (scan_pair_kernel):
 // the intermediate table (A's output, B's input) stays in registers.  Rows of that
 // table fall into groups, cosets q0 + W of a subspace W (dim <= 3) closed under A's
@@ -108,6 +130,7 @@ struct Plan {
   int rmax = 0;
   // Derived execution data (valid when executable()).
   std::vector<DevStep> dev;
+  std::vector<ResStep> res;                // on-chip step records (rmax <= kResMaxRank, else empty)
   std::vector<unsigned long long> tables;  // concatenated byte tables
   // Fused pairs: pair_at[j] >= 0 when positions j and j + 1 run as pairs[pair_at[j]].
   std::vector<DevPair> pairs;
@@ -118,7 +141,7 @@ struct Plan {
   // Device copies, per device ordinal (created lazily by the executor).
   struct DeviceCopy {
     int device = -1;
-    void* steps = nullptr;    // DevStep[n]
+    void* res = nullptr;      // ResStep[n] (plans of rank <= kResMaxRank)
     void* tables = nullptr;   // u64[tables.size()]
     void* verts = nullptr;    // DevVert[n]
   };

@@ -29,7 +29,7 @@ Plan::~Plan() {
   for (auto& d : device_copies) {
     if (d.device < 0) continue;
     cudaSetDevice(d.device);
-    if (d.steps) cudaFree(d.steps);
+    if (d.res) cudaFree(d.res);
     if (d.tables) cudaFree(d.tables);
     if (d.verts) cudaFree(d.verts);
   }
@@ -83,10 +83,12 @@ int plan_device_copy(Plan& plan, int device, const Plan::DeviceCopy** out) {
     verts[j].fixed = plan.steps[j].free ? 0 : 1;
   }
   const size_t tb = std::max<size_t>(1, plan.tables.size()) * sizeof(unsigned long long);
-  RGS_CUDA_TRY(cudaMalloc(&d.steps, sizeof(DevStep) * plan.n));
+  if (!plan.res.empty()) {
+    RGS_CUDA_TRY(cudaMalloc(&d.res, sizeof(ResStep) * plan.n));
+    RGS_CUDA_TRY(cudaMemcpy(d.res, plan.res.data(), sizeof(ResStep) * plan.n, cudaMemcpyHostToDevice));
+  }
   RGS_CUDA_TRY(cudaMalloc(&d.tables, tb));
   RGS_CUDA_TRY(cudaMalloc(&d.verts, sizeof(DevVert) * plan.n));
-  RGS_CUDA_TRY(cudaMemcpy(d.steps, plan.dev.data(), sizeof(DevStep) * plan.n, cudaMemcpyHostToDevice));
   if (!plan.tables.empty())
     RGS_CUDA_TRY(cudaMemcpy(d.tables, plan.tables.data(), plan.tables.size() * sizeof(unsigned long long),
                             cudaMemcpyHostToDevice));
