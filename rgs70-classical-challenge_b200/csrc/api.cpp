@@ -275,7 +275,7 @@ int rgs_chain_launch_count(const rgs_plan* plan, int64_t count, int32_t batch_ti
                            int32_t with_logp, int64_t* launches) {
   if (!plan || !launches) return fail(RGS_ERR_ARG, "null argument");
   if (count < 0 || batch_tile < 1) return fail(RGS_ERR_ARG, "count must be >= 0 and batch_tile >= 1");
-  *launches = (count + batch_tile - 1) / batch_tile * chain_launches_per_tile(plan->plan, marginals != 0, with_logp != 0);
+  *launches = chain_launches(plan->plan, count, batch_tile, marginals != 0, with_logp != 0);
   return RGS_OK;
 }
 

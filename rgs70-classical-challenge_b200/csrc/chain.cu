@@ -21,6 +21,11 @@
 // positions never reaches memory: per pair 2 reads of j's input and 1 write instead of 1
 // read, 3 passes over the intermediate table and 1 write.
 // The final table is the amplitude of the drawn string, returned like rgs_scan_amplitudes.
+//
+// Plans of rank <= kResPlanRank run on chip instead (resident.cu): one launch for the
+// whole call, tables in shared memory.  Streamed, such a plan is all launches -- per 128
+// strings about three per position, none of them filling the GPU (n = 56, rank 9, 8192
+// strings: 23,400 launches, 53 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -30,6 +35,7 @@
 #include "chain.hpp"
 #include "philox.cuh"
 #include "plan.hpp"
+#include "resident.hpp"
 #include "scan.hpp"
 #include "scan_device.cuh"
 #include "scan_row.cuh"
@@ -370,6 +376,18 @@ long long chain_launches_per_tile(const Plan& plan, bool mode_given, bool with_l
   return c + 1;
 }
 
+// Strings of one on-chip launch, or 0 where the plan is streamed.
+long long chain_onchip_strings(const Plan& plan, long long count, int Bt) {
+  if (!plan.fuse || !resident_plan_fits(plan)) return 0;
+  return Bt >= kChainMaxTile / 2 ? std::max<long long>(count, 1) : Bt;
+}
+
+long long chain_launches(const Plan& plan, long long count, int Bt, bool mode_given, bool with_logp) {
+  const long long per = chain_onchip_strings(plan, count, Bt);
+  if (per) return (count + per - 1) / per;
+  return (count + Bt - 1) / Bt * chain_launches_per_tile(plan, mode_given, with_logp);
+}
+
 int chain_run(Plan& plan, const double* U, long long count, int mode_given, u64 seed, const double* uniforms,
               int precision, unsigned long long* bits, void* out_value, double* out_logscale, double* out_logp,
               float* out_cond1, void* workspace, size_t ws_bytes, int Bt, cudaStream_t stream, bool check) {
@@ -398,6 +416,34 @@ int chain_run(Plan& plan, const double* U, long long count, int mode_given, u64 
   // Fused pairs of positions (the plan's pairs), every precision.
   const bool fuse = !plan.pair_at.empty();
   RGS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), stream));
+  auto finish = [&]() -> int {
+    if (!check) return RGS_OK;
+    int h = 0;
+    RGS_CUDA_TRY(cudaMemcpyAsync(&h, status, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    RGS_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (h) return fail(RGS_ERR_ZERO_NORM, "a branch pair had zero or non-finite total mass");
+    return RGS_OK;
+  };
+  const long long onchip = chain_onchip_strings(plan, count, Bt);
+  if (onchip) {
+    const size_t vsize = precision == RGS_PREC_C128 ? 16 : 8;
+    for (long long first = 0; first < count; first += onchip) {
+      ResInstance in{};
+      in.U = U;
+      in.count = std::min(onchip, count - first);
+      in.seed = seed;
+      in.item0 = first;
+      in.uniforms = uniforms ? uniforms + (size_t)first * plan.n : nullptr;
+      in.bits = bits + 2 * first;
+      in.sample_bits = bits + 2 * first;
+      in.out_value = in.sample_value = (char*)out_value + (size_t)first * vsize;
+      in.out_logscale = in.sample_logscale = out_logscale + first;
+      in.sample_logp = out_logp ? out_logp + first : nullptr;
+      in.out_cond = out_cond1 ? out_cond1 + (size_t)first * plan.n : nullptr;
+      if ((rc = resident_run_plan(plan, *dc, mode_given ? 2 : 1, precision, in, device, status, stream))) return rc;
+    }
+    return finish();
+  }
   for (long long first = 0; first < count; first += Bt) {
     const int cnt = (int)std::min<long long>(Bt, count - first);
     if (!mode_given) chain_clear_bits_kernel<<<(cnt + 127) / 128, 128, 0, stream>>>(bits, first, cnt);
@@ -452,13 +498,7 @@ int chain_run(Plan& plan, const double* U, long long count, int mode_given, u64 
                                       (char*)out_value + (size_t)first * (precision == RGS_PREC_C128 ? 16 : 8),
                                       out_logscale + first, stream));
   }
-  if (check) {
-    int h = 0;
-    RGS_CUDA_TRY(cudaMemcpyAsync(&h, status, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    RGS_CUDA_TRY(cudaStreamSynchronize(stream));
-    if (h) return fail(RGS_ERR_ZERO_NORM, "a branch pair had zero or non-finite total mass");
-  }
-  return RGS_OK;
+  return finish();
 }
 
 }  // namespace rgs
