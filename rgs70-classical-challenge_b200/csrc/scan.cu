@@ -17,6 +17,7 @@
 
 #include "common.hpp"
 #include "plan.hpp"
+#include "resident.hpp"
 #include "scan.hpp"
 #include "scan_device.cuh"
 #include "scan_row.cuh"
@@ -479,6 +480,12 @@ int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, Ch
   return RGS_OK;
 }
 
+bool scan_on_chip(const Plan& plan, int precision, long long batch) {
+  if (!plan.fuse || !resident_plan_fits(plan)) return false;
+  if (batch > kOnChipFew && batch < kOnChipMany) return false;
+  return precision != RGS_PREC_C128 || plan.rmax <= 10 || batch <= 1024;
+}
+
 int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, size_t ws_bytes, long long* out) {
   if (batch < 0) return fail(RGS_ERR_ARG, "batch must be >= 0");
   ScanLayout L;
@@ -489,7 +496,9 @@ int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, 
   if ((rc = scan_pick_chunk(plan, Bt, precision, ws_bytes, C, &S))) return rc;
   const long long n = plan.n;
   long long total = 0;
-  if (S < 2) {
+  if (scan_on_chip(plan, precision, batch)) {
+    total = batch ? 1 : 0;
+  } else if (S < 2) {
     total = (batch + Bt - 1) / Bt * ((long long)segments_of(plan, 0, (int)n).size() + 2);
   } else {
     const long long stride = (long long)S * Bt;
@@ -508,6 +517,35 @@ int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, 
 }
 
 namespace {
+
+// The whole batch as one on-chip launch.  The workspace is not used, but what the streamed
+// sweep refuses is refused here too.
+int scan_run_on_chip(Plan& plan, const double* U, const u64* bits, const double* fvec, long long batch, int precision,
+                     void* out_value, double* out_logscale, void* workspace, size_t ws_bytes, int Bt,
+                     cudaStream_t stream, ScanStats* stats) {
+  ScanLayout L;
+  int rc = scan_layout(plan, Bt, precision, L);
+  if (rc) return rc;
+  if (ws_bytes < L.total()) return fail(RGS_ERR_OOM, "workspace smaller than one tile's layout (rgs_scan_workspace_bytes)");
+  if (((uintptr_t)workspace & 255) != 0) return fail(RGS_ERR_ARG, "workspace must be 256-byte aligned");
+  int device = 0;
+  rc = bind_device_of(workspace, &device);
+  if (rc) return rc;
+  const Plan::DeviceCopy* dc = nullptr;
+  rc = plan_device_copy(plan, device, &dc);
+  if (rc) return rc;
+  ResInstance in{};
+  in.U = U;
+  in.fvec = fvec;
+  in.bits = fvec ? nullptr : bits;
+  in.count = batch;
+  in.out_value = out_value;
+  in.out_logscale = out_logscale;
+  rc = resident_run_plan(plan, *dc, 0, precision, in, device, nullptr, stream);
+  if (rc) return rc;
+  if (stats) stats->launches = 1;
+  return RGS_OK;
+}
 
 // Tile-by-tile sweep (every position, one launch per tile): the path for workspaces sized
 // by scan_layout alone.
@@ -580,6 +618,9 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
   int S = 0;
   int rc = scan_pick_chunk(plan, Bt, precision, ws_bytes, C, &S);
   if (rc) return rc;
+  if (scan_on_chip(plan, precision, batch))
+    return scan_run_on_chip(plan, U, bits, fvec, batch, precision, out_value, out_logscale, workspace, ws_bytes, Bt,
+                            stream, stats);
   if (S < 2)
     return scan_run_tiles(plan, U, bits, fvec, batch, precision, out_value, out_logscale, workspace, ws_bytes, Bt,
                           stream, stats);

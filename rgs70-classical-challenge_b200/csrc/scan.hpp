@@ -41,6 +41,16 @@ int scan_chunk_tiles(int Bt);
 // Tiles per chunk that scan_run uses with a workspace of ws_bytes (the largest S <=
 // scan_chunk_tiles(Bt), S >= 2, whose layout fits, with C filled in); 0: tile by tile.
 int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, ChunkLayout& C, int* S);
+// Whether scan_run sweeps `batch` strings of a plan on chip, as one launch (resident.cu),
+// instead of one launch per position: plans of rank <= kResPlanRank with fusion on.
+// Measured, on chip against streamed: one string 31 against 166 us (rank 9, n = 40), 300
+// strings 44 against 266 us (rank 10), 8192 strings 183 against 422 us (rank 10, complex64,
+// float32 arithmetic), 975 against 1210 us (rank 12); complex128 at rank 11: 181 against
+// 295 us for 1000 strings, but 1026 against 836 us for 8192 (three units per SM: too few
+// warps), so large complex128 batches above rank 10 are streamed.  Sweeps of 33 to 127
+// strings keep the position-by-position launch schedule of one tile.
+constexpr long long kOnChipFew = 32, kOnChipMany = 128;
+bool scan_on_chip(const Plan& plan, int precision, long long batch);
 // Kernel launches scan_run queues for `batch` items with that workspace.
 int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, size_t ws_bytes, long long* out);
 
