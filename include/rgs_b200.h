@@ -334,7 +334,7 @@ int rgs_gemm_bf16(int32_t M, int32_t N, int32_t K, const void* A, int32_t lda, i
  * results are then invalid); clears the flag.
  * Synchronous. */
 int rgs_tensor_core_status(int32_t* timed_out);
-/* TMA loads of the GEMM's K-major operands with 16-byte aligned rows: on (1, default) or
+/* TMA loads of the GEMM's operands with 16-byte aligned rows: on (1, default) or
  * off (0: every operand staged by the threads).  Both paths issue the same MMAs in the
  * same order; the switch exists for tests and measurements.  Process-wide. */
 int rgs_gemm_set_tma(int32_t on);

@@ -106,7 +106,6 @@ int rgs_mlp_bwd(int32_t batch, int32_t n, int32_t hidden, const void* x, const v
   g.C = gw3;
   g.ldc = hidden;
   if ((rc = gemm_bf16(g, s))) return rc;
-  if ((rc = colsum_bf16((cbf)dzb, batch, n, gb3, s))) return rc;
   g = make(batch, hidden, n, dzb, n, 0, w3b, hidden, 0);  // dh2 = dz W3 * [h2 > 0]
   g.gate = (cbf)h2b;
   g.Cb = (bf)dh2b;
@@ -117,7 +116,6 @@ int rgs_mlp_bwd(int32_t batch, int32_t n, int32_t hidden, const void* x, const v
   g.C = gw2;
   g.ldc = hidden;
   if ((rc = gemm_bf16(g, s))) return rc;
-  if ((rc = colsum_bf16((cbf)dh2b, batch, hidden, gb2, s))) return rc;
   g = make(batch, hidden, hidden, dh2b, hidden, 0, w2b, hidden, 0);  // dh1 = dh2 W2 * [h1 > 0]
   g.gate = (cbf)h1b;
   g.Cb = (bf)dh1b;
@@ -128,7 +126,10 @@ int rgs_mlp_bwd(int32_t batch, int32_t n, int32_t hidden, const void* x, const v
   g.C = gw1;
   g.ldc = n;
   if ((rc = gemm_bf16(g, s))) return rc;
-  return colsum_bf16((cbf)dh1b, batch, hidden, gb1, s);
+  const cbf grads[3] = {(cbf)dzb, (cbf)dh2b, (cbf)dh1b};  // bias gradients
+  const int cols[3] = {n, hidden, hidden};
+  float* const gb[3] = {gb3, gb2, gb1};
+  return colsum3_bf16(grads, cols, gb, batch, s);
 }
 
 int rgs_mlp_adam(float* w, const float* grad, float* m1, float* m2, const uint8_t* mask, void* wb, int32_t count,

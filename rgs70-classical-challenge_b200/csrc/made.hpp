@@ -22,13 +22,14 @@ struct GemmArgs {
 };
 
 int gemm_bf16(const GemmArgs& g, cudaStream_t s);
-// TMA loads of the K-major aligned GEMM operands on (1, default) or off (0).
+// TMA loads of the aligned GEMM operands on (1, default) or off (0).
 int gemm_set_tma(int on);
 // Reads and clears the flag that a bounded tensor-core wait gave up (synchronous).
 int tensor_core_status(int* timed_out);
 int bce_grad(const float* z, const float* target, int count, float scale, __nv_bfloat16* dz, double* partial,
              int blocks, cudaStream_t s);
-int colsum_bf16(const __nv_bfloat16* x, int rows, int cols, float* out, cudaStream_t s);
+// Column sums of three bf16 matrices [rows][cols[k]] in one launch.
+int colsum3_bf16(const __nv_bfloat16* const x[3], const int cols[3], float* const out[3], int rows, cudaStream_t s);
 int adam_step(float* w, const float* grad, float* m1, float* m2, const unsigned char* mask, __nv_bfloat16* wb,
               int count, float lr, float b1, float b2, float eps, int t, cudaStream_t s);
 int sample_position(const float* z, int n, int d, int count, unsigned long long seed, unsigned long long first,

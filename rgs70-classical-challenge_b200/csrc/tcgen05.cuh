@@ -11,6 +11,9 @@
 //    box 64 elements wide): rows 128 bytes apart, SBO = 1024 (eight rows); the k-th
 //    16-element slice of a row starts 32 * k bytes further (the swizzle is applied by the
 //    hardware from the address bits, so the tile must be 1024-byte aligned).
+//  * MN-major, 128-byte swizzle (boxes 64 elements of M or N wide): the k-rows of a box are
+//    128 bytes apart, SBO = 1024 (eight k-rows), LBO = byte distance of the next 64
+//    elements of M or N; the k-th 16-row slice starts 2048 * k bytes further.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -69,6 +72,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   for (uint32_t i = 0; i < kWaitLimit; ++i)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
+}
+
+// ------------------------------------------------------------------ clusters
+// Barrier of every thread of the cluster (release / acquire: shared-memory writes before
+// it are visible to the peers after it).
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();  // the barrier is a warp-converged instruction
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// 16 bytes of the shared memory of block `rank` of the cluster, at this block's address p.
+__device__ __forceinline__ float4 ld_cluster_f4(const void* p, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
 }
 
 // ------------------------------------------------------------------ TMEM
