@@ -376,15 +376,15 @@ long long chain_launches_per_tile(const Plan& plan, bool mode_given, bool with_l
   return c + 1;
 }
 
-// Strings of one on-chip launch, or 0 where the plan is streamed.
-long long chain_onchip_strings(const Plan& plan, long long count, int Bt) {
-  if (!plan.fuse || !resident_plan_fits(plan)) return 0;
-  return Bt >= kChainMaxTile / 2 ? std::max<long long>(count, 1) : Bt;
+// Whether chain_run takes a plan on chip: rank <= kResPlanRank, fusion on, and a tile of 64
+// (the largest of complex128) or more.  A caller that asks for smaller tiles bounds the
+// strings in flight and keeps the streamed schedule, one launch sequence per tile.
+bool chain_on_chip(const Plan& plan, int Bt) {
+  return plan.fuse && resident_plan_fits(plan) && Bt >= kChainMaxTile / 2;
 }
 
 long long chain_launches(const Plan& plan, long long count, int Bt, bool mode_given, bool with_logp) {
-  const long long per = chain_onchip_strings(plan, count, Bt);
-  if (per) return (count + per - 1) / per;
+  if (chain_on_chip(plan, Bt)) return count ? 1 : 0;
   return (count + Bt - 1) / Bt * chain_launches_per_tile(plan, mode_given, with_logp);
 }
 
@@ -424,24 +424,18 @@ int chain_run(Plan& plan, const double* U, long long count, int mode_given, u64 
     if (h) return fail(RGS_ERR_ZERO_NORM, "a branch pair had zero or non-finite total mass");
     return RGS_OK;
   };
-  const long long onchip = chain_onchip_strings(plan, count, Bt);
-  if (onchip) {
-    const size_t vsize = precision == RGS_PREC_C128 ? 16 : 8;
-    for (long long first = 0; first < count; first += onchip) {
-      ResInstance in{};
-      in.U = U;
-      in.count = std::min(onchip, count - first);
-      in.seed = seed;
-      in.item0 = first;
-      in.uniforms = uniforms ? uniforms + (size_t)first * plan.n : nullptr;
-      in.bits = bits + 2 * first;
-      in.sample_bits = bits + 2 * first;
-      in.out_value = in.sample_value = (char*)out_value + (size_t)first * vsize;
-      in.out_logscale = in.sample_logscale = out_logscale + first;
-      in.sample_logp = out_logp ? out_logp + first : nullptr;
-      in.out_cond = out_cond1 ? out_cond1 + (size_t)first * plan.n : nullptr;
-      if ((rc = resident_run_plan(plan, *dc, mode_given ? 2 : 1, precision, in, device, status, stream))) return rc;
-    }
+  if (chain_on_chip(plan, Bt)) {
+    ResInstance in{};
+    in.U = U;
+    in.count = count;
+    in.seed = seed;
+    in.uniforms = uniforms;
+    in.bits = in.sample_bits = bits;
+    in.out_value = in.sample_value = out_value;
+    in.out_logscale = in.sample_logscale = out_logscale;
+    in.sample_logp = out_logp;
+    in.out_cond = out_cond1;
+    if ((rc = resident_run_plan(plan, *dc, mode_given ? 2 : 1, precision, in, device, status, stream))) return rc;
     return finish();
   }
   for (long long first = 0; first < count; first += Bt) {

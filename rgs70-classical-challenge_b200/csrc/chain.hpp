@@ -20,9 +20,8 @@ int chain_layout(const Plan& plan, int Bt, int precision, ChainLayout& L);
 // Kernel launches of chain_run per batch tile (sampling: mode_given = false).
 long long chain_launches_per_tile(const Plan& plan, bool mode_given, bool with_logp);
 
-// Kernel launches of one chain_run call.  A plan that runs on chip takes one launch per
-// call, or one per Bt strings where the caller asked for a tile below 64 (the largest tile
-// of complex128), which bounds the strings in flight.
+// Kernel launches of one chain_run call: one for plans that run on chip (rank <=
+// kResPlanRank, tile >= 64).
 long long chain_launches(const Plan& plan, long long count, int Bt, bool mode_given, bool with_logp);
 
 // mode_given = 0: draw x (Philox(seed) uniforms, or `uniforms` [count][n] in scan

