@@ -63,13 +63,14 @@ def build_instance_cpu():
                                              target_rank=TARGET_RANK, order_seeds=ORDER_SEEDS)
 
 
-def step_bytes(ranks, esize, pairs=()):
-    """Compulsory table traffic of one sweep: every input entry read once, every output
-    written once (step 0 reads the implicit unit table); a fused pair (j, j + 1) neither
-    writes nor reads the table between its two positions."""
+def step_bytes(ranks, esize, segments=None):
+    """Compulsory table traffic of one sweep: every pass reads its input once and writes its
+    output once (position 0 reads the implicit unit table).  segments: the sweep's passes as
+    (first position, positions); the tables inside a pass do not reach memory.  Default: one
+    position per pass."""
     r_in = [0] + list(ranks[:-1])
-    total = sum((1 << a) * (j > 0) + (1 << b) for j, (a, b) in enumerate(zip(r_in, ranks)))
-    return esize * (total - sum(2 << ranks[j] for j in pairs))
+    segments = segments if segments is not None else [(j, 1) for j in range(len(ranks))]
+    return esize * sum((1 << r_in[j]) * (j > 0) + (1 << ranks[j + k - 1]) for j, k in segments)
 
 
 def chain_bytes(plan, esize, fused=True):
@@ -471,8 +472,8 @@ def run_ours(args, rank, world, local_rank):
 
     # Roofline of the scan-step kernels (dominant: every launch but the weights and
     # finalisation kernels, one or two per chunk of tiles).
-    b64 = step_bytes(inst.ranks, 8, plan.pairs) * BATCH if use64 else 0
-    b128 = step_bytes(inst.ranks, 16, plan.pairs) * BATCH if use128 else 0
+    b64 = step_bytes(inst.ranks, 8, plan.segments) * BATCH if use64 else 0
+    b128 = step_bytes(inst.ranks, 16, plan.segments) * BATCH if use128 else 0
     peaks_path = ROOT / "MEASURED_PEAKS.json"
     peak, peak_src = 6650.0, "fallback"
     if peaks_path.exists():
@@ -928,7 +929,7 @@ def run_rgs70(args, rank, world, local_rank):
             esize = 16 if prec == "c128" else 8
             legs[prec] = {"amplitudes_per_s": len(bits) * args.steps / t, "batch_tile": tile,
                           "max_rel_err_vs_reference_c128": float(np.max(np.abs(p - ref_p) / ref_p)),
-                          "achieved_GBps": step_bytes(plan_f.ranks, esize, plan_f.pairs) * len(bits) * args.steps
+                          "achieved_GBps": step_bytes(plan_f.ranks, esize, plan_f.segments) * len(bits) * args.steps
                           / t / 1e9,
                           "launches_per_sweep": eng.launch_count(len(bits))}
             del eng, val, ls

@@ -86,6 +86,11 @@ int rgs_plan_set_fusion(rgs_plan* plan, int32_t on);
 /* Number of fused pairs and (if first_positions is not NULL) position j of each,
  * int32[count]. */
 int rgs_plan_pairs(const rgs_plan* plan, int32_t* count, int32_t* first_positions);
+/* The passes over memory of a streamed sweep (one position, a fused pair, or a run of
+ * positions whose interior tables stay on chip: middle positions of plans of rank 18 and
+ * above): first position and number of positions of each, int32[count] (at most n;
+ * either array may be NULL). */
+int rgs_plan_segments(const rgs_plan* plan, int32_t* count, int32_t* first_positions, int32_t* lengths);
 /* Pair record k for inspection: the GF(2) data the pair kernel runs on.  Codes:
  * 0 PAIR 1 combo, 1 PAIR 2 combos (second with y bit 1), 2 PAIR 2 combos (both y bit 0),
  * 3 PAIR 4 combos (two with y bit 1), 4 MERGE 2 combos. */

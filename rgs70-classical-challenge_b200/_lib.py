@@ -70,6 +70,7 @@ SIGNATURES = {
                                         c_int32_p]),
     "rgs_plan_set_fusion": (ctypes.c_int, [c_void_p, ctypes.c_int32]),
     "rgs_plan_pairs": (ctypes.c_int, [c_void_p, c_int32_p, c_int32_p]),
+    "rgs_plan_segments": (ctypes.c_int, [c_void_p, c_int32_p, c_int32_p, c_int32_p]),
     "rgs_plan_pair_info": (ctypes.c_int, [c_void_p, ctypes.c_int32, c_void_p]),
     "rgs_scan_workspace_bytes": (ctypes.c_int, [c_void_p, ctypes.c_int32, ctypes.c_int32, c_size_t_p]),
     "rgs_scan_launch_count": (ctypes.c_int, [c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32,

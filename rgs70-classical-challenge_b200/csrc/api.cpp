@@ -134,6 +134,19 @@ int rgs_plan_pairs(const rgs_plan* plan, int32_t* count, int32_t* first_position
   return RGS_OK;
 }
 
+int rgs_plan_segments(const rgs_plan* plan, int32_t* count, int32_t* first_positions, int32_t* lengths) {
+  if (!plan || !count) return fail(RGS_ERR_ARG, "null argument");
+  if (!plan->plan.exec_ok) return fail(RGS_ERR_UNSUPPORTED, plan->plan.exec_reason);
+  std::vector<int> first, length;
+  scan_segments(plan->plan, first, length);
+  *count = (int32_t)first.size();
+  for (size_t k = 0; k < first.size(); ++k) {
+    if (first_positions) first_positions[k] = first[k];
+    if (lengths) lengths[k] = length[k];
+  }
+  return RGS_OK;
+}
+
 int rgs_plan_pair_info(const rgs_plan* plan, int32_t k, rgs_pair_info* info) {
   if (!plan || !info) return fail(RGS_ERR_ARG, "null argument");
   if (k < 0 || k >= (int32_t)plan->plan.pairs.size()) return fail(RGS_ERR_ARG, "pair index out of range");

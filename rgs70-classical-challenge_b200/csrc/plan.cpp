@@ -362,6 +362,258 @@ void build_pairs(Plan& p) {
   p.tables.insert(p.tables.end(), mb.begin(), mb.end());
 }
 
+// A subspace as a reduced echelon basis (highest-bit pivots, each pivot in one vector).
+struct Subspace {
+  std::vector<u128> basis;
+  std::vector<int> piv;
+  bool add(u128 v) {
+    for (size_t i = 0; i < basis.size(); ++i)
+      if (bit_of(v, piv[i])) v ^= basis[i];
+    if (!v) return false;
+    const int h = highest_bit(v);
+    for (auto& b : basis)
+      if (bit_of(b, h)) b ^= v;
+    basis.push_back(v);
+    piv.push_back(h);
+    return true;
+  }
+  int dim() const { return (int)basis.size(); }
+  // Coordinates of v; false when v lies outside.
+  bool coords(u128 v, unsigned& c) const {
+    c = 0;
+    for (size_t i = 0; i < basis.size(); ++i)
+      if (bit_of(v, piv[i])) {
+        c |= 1u << i;
+        v ^= basis[i];
+      }
+    return !v;
+  }
+  u128 at(unsigned c) const {
+    u128 v = 0;
+    for (size_t i = 0; i < basis.size(); ++i)
+      if ((c >> i) & 1) v ^= basis[i];
+    return v;
+  }
+};
+
+// The record of the run [j, j + k), or false when its closed subspaces are too large.
+// Appends the run's tables (u64 words, offsets relative to the end of p.tables).
+bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned long long>* words_out) {
+  if (k < 2 || k > kBlockLen || j < 1 || j + k > p.n) return false;
+  for (int i = 0; i < k; ++i) {
+    const PlanStep& st = p.steps[j + i];
+    if (!st.free || st.r_in > 31 || st.r_out > 31) return false;
+  }
+  auto cmask = [&](int i) { return one_at(p.steps[j + i].r_in) - 1; };
+  std::vector<Subspace> D(k + 1);
+  const int limit = std::max(kBlockDim, kBlockEnds);
+  for (bool changed = true; changed;) {
+    changed = false;
+    for (int i = 0; i < k; ++i) {
+      const PlanStep& st = p.steps[j + i];
+      if (st.ycol) changed |= D[i + 1].add(st.ycol);
+      for (size_t b = 0; b < D[i].basis.size(); ++b) changed |= D[i + 1].add(apply_cols(st.mcols, D[i].basis[b]));
+    }
+    for (int i = k - 1; i >= 0; --i) {
+      const PlanStep& st = p.steps[j + i];
+      for (u128 v : st.kernel) changed |= D[i].add(v & cmask(i));
+      for (size_t b = 0; b < D[i + 1].basis.size(); ++b)
+        changed |= D[i].add(apply_cols(st.lcols, D[i + 1].basis[b]) & cmask(i));
+    }
+    for (auto& d : D)
+      if (d.dim() > limit) return false;
+  }
+  DevBlock d{};
+  d.j = j;
+  d.k = k;
+  d.r_in = p.steps[j].r_in;
+  d.r_out = p.steps[j + k - 1].r_out;
+  d.din = D[0].dim();
+  d.dout = D[k].dim();
+  d.dmax = 0;
+  for (int i = 1; i < k; ++i) d.dmax = std::max(d.dmax, D[i].dim());
+  if (d.din > kBlockEnds || d.dout > kBlockEnds || d.dmax > kBlockDim) return false;
+  d.lg = d.r_out - d.dout;
+  if (!words_out) return true;  // feasible; the tables are built for chosen runs only
+  std::vector<unsigned long long>& words = *words_out;
+  auto parity = [](u128 x) {
+    return (__builtin_popcountll((uint64_t)x) + __builtin_popcountll((uint64_t)(x >> 64))) & 1;
+  };
+  // Slots of the interior levels: linear images of the local basis vectors.
+  std::vector<std::vector<unsigned>> slot(k + 1);
+  auto slot_of = [&](int i, unsigned c) {
+    unsigned s = 0;
+    for (size_t b = 0; b < slot[i].size(); ++b)
+      if ((c >> b) & 1) s ^= slot[i][b];
+    return s;
+  };
+  std::vector<unsigned long long> prog;
+  for (int i = 0; i < k; ++i) {
+    const PlanStep& st = p.steps[j + i];
+    const DevStep& ds = p.dev[j + i];
+    const bool pair = ds.mode == MODE_PAIR;
+    unsigned tloc = 0;
+    if (pair && !D[i + 1].coords(st.ycol, tloc)) return false;
+    int pivot = -1;  // row operations of a pair: the local rows without this coordinate
+    if (pair)
+      for (int b = 0; b < D[i + 1].dim(); ++b)
+        if ((tloc >> b) & 1) pivot = b;
+    // Slots of level i + 1.
+    if (i == 0) {
+      for (int b = 0; b < D[1].dim(); ++b) slot[1].push_back(1u << b);
+    } else if (i + 1 < k) {
+      unsigned tslot = 0;  // slot offset of a pair's second output
+      if (pair) {
+        for (u128 v : st.kernel) {
+          unsigned c = 0;
+          if (!tslot && (v & cmask(i)) && D[i].coords(v & cmask(i), c)) tslot = slot_of(i, c);
+        }
+        if (!tslot) {  // growth: the lowest slot bit outside the level's span
+          Subspace span;
+          for (unsigned s : slot[i]) span.add(s);
+          for (int b = 0; b < kBlockDim && !tslot; ++b) {
+            Subspace t = span;
+            if (t.add(one_at(b))) tslot = 1u << b;
+          }
+          if (!tslot) return false;
+        }
+      }
+      slot[i + 1].assign(D[i + 1].dim(), 0);
+      for (int b = 0; b < D[i + 1].dim(); ++b) {
+        if (b == pivot) continue;
+        unsigned c = 0;
+        if (!D[i].coords(apply_cols(st.lcols, D[i + 1].at(1u << b)) & cmask(i), c)) return false;
+        slot[i + 1][b] = slot_of(i, c);
+      }
+      if (pair) {
+        // t = pivot vector + others of tloc: the pivot's slot follows from t's.
+        unsigned s = tslot;
+        for (int b = 0; b < D[i + 1].dim(); ++b)
+          if (b != pivot && ((tloc >> b) & 1)) s ^= slot[i + 1][b];
+        slot[i + 1][pivot] = s;
+      }
+    }
+    const bool last = i + 1 == k;
+    auto place = [&](unsigned c) { return last ? c : slot_of(i + 1, c); };
+    d.code[i] = pair ? (ds.ncombos == 1 ? RC_P1
+                                        : (ds.ncombos == 2 ? (ds.ng0 == 2 ? RC_P2F : RC_P2H)
+                                                           : (ds.ng0 == 4 ? RC_P4F : RC_P4H)))
+                     : (ds.ncombos == 1 ? RC_M1 : RC_M2);
+    d.first[i] = (int)prog.size();
+    d.pair[i] = pair ? (int)place(tloc) : 0;
+    d.rows[i] = 0;
+    for (unsigned c = 0; c < (1u << D[i + 1].dim()); ++c) {
+      if (pair && ((c >> pivot) & 1)) continue;
+      const u128 l0 = apply_cols(st.lcols, D[i + 1].at(c));
+      const unsigned y0 = pair ? (unsigned)bit_of(l0, st.r_in) : 0u;
+      unsigned long long w = (unsigned long long)place(y0 ? c ^ tloc : c) << 32;
+      for (int q = 0; q < ds.ncombos; ++q) {
+        const u128 cc = (l0 ^ (u128)ds.combos[q]) & cmask(i);
+        unsigned in = 0;
+        if (!D[i].coords(cc, in)) return false;
+        w |= (unsigned long long)(i == 0 ? in : slot_of(i, in)) << (8 * q);
+        w |= (unsigned long long)parity(cc & st.beta) << (40 + q);
+      }
+      prog.push_back(w);
+      ++d.rows[i];
+    }
+  }
+  d.words = (int)prog.size();
+  // Group maps of every group-index bit, then byte tables.
+  std::vector<unsigned long long> rows_of(d.lg), flags_of(d.lg);
+  int bit = 0;
+  for (int pos = 0; pos < d.r_out; ++pos) {
+    if (std::find(D[k].piv.begin(), D[k].piv.end(), pos) != D[k].piv.end()) continue;
+    u128 x = one_at(pos);
+    unsigned long long flags = 0;
+    const unsigned long long outrow = (unsigned long long)x;
+    for (int i = k - 1; i >= 0; --i) {
+      const PlanStep& st = p.steps[j + i];
+      const u128 q = apply_cols(st.lcols, x);
+      x = q & cmask(i);
+      flags |= (unsigned long long)bit_of(q, st.r_in) << (2 * i);
+      flags |= (unsigned long long)parity(x & st.beta) << (2 * i + 1);
+    }
+    rows_of[bit] = (unsigned long long)x | (outrow << 32);
+    flags_of[bit] = flags;
+    ++bit;
+  }
+  d.nbytes = (d.lg + 7) / 8;
+  if ((p.tables.size() + words.size()) & 1) words.push_back(0ull);
+  d.tab_off = p.tables.size() + words.size();
+  for (int b = 0; b < d.nbytes; ++b)
+    for (int v = 0; v < 256; ++v) {
+      unsigned long long r = 0, f = 0;
+      for (int q = 0; q < 8 && 8 * b + q < d.lg; ++q)
+        if ((v >> q) & 1) {
+          r ^= rows_of[8 * b + q];
+          f ^= flags_of[8 * b + q];
+        }
+      words.push_back(r);
+      words.push_back(f);
+    }
+  d.prog_off = p.tables.size() + words.size();
+  words.insert(words.end(), prog.begin(), prog.end());
+  d.lin_off = p.tables.size() + words.size();
+  std::vector<unsigned> lin;
+  for (unsigned c = 0; c < (1u << d.din); ++c) lin.push_back((unsigned)D[0].at(c));
+  for (unsigned c = 0; c < (1u << d.dout); ++c) lin.push_back((unsigned)D[k].at(c));
+  if (lin.size() & 1) lin.push_back(0u);
+  for (size_t i = 0; i < lin.size(); i += 2) words.push_back((unsigned long long)lin[i] | ((unsigned long long)lin[i + 1] << 32));
+  out = d;
+  return true;
+}
+
+// Chooses the runs of the middle positions (plans of rank >= kBlockRank): segments of one
+// position, one fused pair or one run, minimising the table entries read and written.
+void build_blocks(Plan& p) {
+  p.blocks.clear();
+  p.block_at.assign(p.n, -1);
+  p.run_len.assign(p.n, 0);
+  if (!p.fuse || !p.exec_ok || p.rmax < kBlockRank || p.rmax > 31) return;
+  for (auto& st : p.steps)
+    if (!st.free) return;
+  int h = 0, t = 0;
+  small_runs(p, h, t);
+  const int lo = std::max(h, 1);
+  if (lo >= t) return;
+  std::vector<double> best(p.n + 1, 0.0);
+  std::vector<int> take(p.n + 1, 1);
+  const double launch = 4096.0;  // entries that one more launch costs, per string
+  for (int j = t - 1; j >= lo; --j) {
+    best[j] = HUGE_VAL;
+    for (int k = 1; k <= kBlockLen && j + k <= t; ++k) {
+      DevBlock d;
+      if (k > 1 && !make_block(p, j, k, d, nullptr)) {
+        // A longer run needs larger subspaces at every level.
+        if (k > 2) break;
+        continue;
+      }
+      const double c = std::ldexp(1.0, p.steps[j].r_in) + std::ldexp(1.0, p.steps[j + k - 1].r_out) + launch + best[j + k];
+      if (c < best[j]) {
+        best[j] = c;
+        take[j] = k;
+      }
+    }
+  }
+  std::vector<unsigned long long> words;
+  for (int j = lo; j < t; j += take[j]) {
+    p.run_len[j] = take[j];
+    // Two positions that the pair kernel covers run there (its rows stay in registers).
+    if (take[j] < 2 || (take[j] == 2 && p.pair_at[j] >= 0)) continue;
+    DevBlock d;
+    if (!make_block(p, j, take[j], d, &words)) {  // not reached: the run was found feasible
+      p.blocks.clear();
+      p.block_at.assign(p.n, -1);
+      p.run_len.assign(p.n, 0);
+      return;
+    }
+    p.block_at[j] = (int)p.blocks.size();
+    p.blocks.push_back(d);
+  }
+  p.tables.insert(p.tables.end(), words.begin(), words.end());
+}
+
 // On-chip step records (plans of rank <= kResMaxRank): see ResStep.
 void build_resident(Plan& p) {
   p.res.clear();
@@ -455,6 +707,7 @@ void build_device(Plan& p) {
   }
   build_resident(p);
   build_pairs(p);
+  build_blocks(p);
 }
 
 }  // namespace
@@ -462,6 +715,7 @@ void build_device(Plan& p) {
 void plan_set_fusion(Plan& p, bool on) {
   p.fuse = on;
   build_pairs(p);
+  build_blocks(p);
 }
 
 std::string compile_plan(int n, const std::vector<std::pair<int, int>>& edges, const std::vector<int>& order,

@@ -116,6 +116,40 @@ struct DevPair {
   int j;                         // position A
 };
 
+// A run of k consecutive free positions j .. j + k - 1 as one pass (scan_block_kernel): the
+// rows of every table of the run fall into groups, cosets of subspaces D_0 (input) .. D_k
+// (output) closed under the run's gathers, so that the rows of one group at one level
+// need only the group's rows of the level before.  A thread carries one string's rows of
+// a group through all k positions in its own shared-memory column.
+// Level i of group g is x_i(g) + D_i, with x_k(g) = g with zeros deposited at the pivots of
+// D_k and x_i the c part of L x_{i+1}; y_i is its y bit and s_i = parity(x_i & beta).  Local
+// rows are coordinates in D_i; the local gathers, signs and destinations do not depend on
+// g except through y_i (swaps a pair's outputs) and s_i (flips every sign).
+// Interior levels live in place: an output row takes the slot of one of its inputs (a
+// growing position adds a slot bit), so a column has 2^dmax slots.
+constexpr int kBlockLen = 6;      // positions per run
+constexpr int kBlockDim = 5;      // dimension of interior levels (32 slots per column)
+constexpr int kBlockEnds = 6;     // dimension of D_0 and D_k
+constexpr int kBlockRank = 18;    // runs are formed in plans of at least this rank
+struct DevBlock {
+  int j, k;
+  int r_in, r_out;
+  int lg, nbytes;                 // log2 groups; byte tables of the group index
+  int din, dout, dmax;
+  int code[kBlockLen];            // ResCode of each position
+  int rows[kBlockLen];            // row operations per group
+  int first[kBlockLen];           // first program word
+  int pair[kBlockLen];            // offset of a pair's second output (slot or local row)
+  int words;                      // program words
+  unsigned long long tab_off;     // u64 index: per (byte, value) the pair (x_0 | x_k << 32,
+                                  // y_i at bit 2 i and s_i at bit 2 i + 1), 16-byte aligned
+  // Program word of a row operation: bits 8 c .. 8 c + 5 the slot (first position: local
+  // input row) of combo c, bits 32..37 the slot (last position: local output row) of the
+  // first output for y_i = 0, bit 40 + c the local sign of combo c.
+  unsigned long long prog_off;
+  unsigned long long lin_off;     // u32 tables: 2^din input rows, then 2^dout output rows
+};
+
 // Positions whose input and output ranks are both at most kSmallRank run once per chunk
 // of tiles (scan.cu); a fused pair never straddles the leading / middle / trailing split.
 constexpr int kSmallRank = 12;
@@ -136,6 +170,11 @@ struct Plan {
   std::vector<DevPair> pairs;
   std::vector<int> pair_at;
   bool fuse = true;                        // build fused pairs (plan_set_fusion)
+  // Runs of positions as one pass: block_at[j] >= 0 when blocks[block_at[j]] starts at j.
+  // run_len[j]: positions of the segment that starts at j (1: alone, 2 without a block: a
+  // fused pair), 0 where no segment starts or outside the middle positions.
+  std::vector<DevBlock> blocks;
+  std::vector<int> block_at, run_len;
   bool exec_ok = false;
   std::string exec_reason;
   // Device copies, per device ordinal (created lazily by the executor).

@@ -424,19 +424,24 @@ cudaError_t scan_launch_pair_gram(int precision, int Bt, int blocks, const DevPa
 
 namespace {
 
-// The sweep as segments: one position, or a fused pair (plan.pair_at).
+// The sweep as segments: one position, a fused pair (plan.pair_at) or a run
+// (plan.block_at, middle positions of large plans).
 struct Segment {
-  int j, len, pair;
+  int j, len, pair, block;
 };
 std::vector<Segment> segments_of(const Plan& plan, int from, int to) {
   std::vector<Segment> out;
   for (int j = from; j < to;) {
+    const int run = plan.blocks.empty() ? 0 : plan.run_len[j];  // 0: not planned as runs
     const int pa = plan.pair_at.empty() ? -1 : plan.pair_at[j];
-    if (pa >= 0 && j + 1 < to) {
-      out.push_back({j, 2, pa});
+    if (run && plan.block_at[j] >= 0) {
+      out.push_back({j, run, -1, plan.block_at[j]});
+      j += run;
+    } else if (pa >= 0 && j + 1 < to && run != 1) {
+      out.push_back({j, 2, pa, -1});
       j += 2;
     } else {
-      out.push_back({j, 1, -1});
+      out.push_back({j, 1, -1, -1});
       j += 1;
     }
   }
@@ -449,6 +454,10 @@ cudaError_t launch_segment(const Plan& plan, const Segment& g, int precision, in
                            const void* Ein, void* Eout, const u64* tables, const double4* W,
                            const unsigned char* F, u64* mx, size_t stride, int tiles, u64 es) {
   const int j = g.j;
+  if (g.block >= 0)  // middle positions: one tile per launch
+    return launch_block(precision, device, s, Ein, Eout, plan.blocks[g.block], tables, W + (size_t)j * stride,
+                        mx + (size_t)(j - 1) * stride, mx + (size_t)j * stride, (int)stride,
+                        __builtin_ctz((unsigned)Bt));
   if (g.len == 2)
     return launch_pair(precision, Bt, device, s, Ein, Eout, plan.pairs[g.pair], tables, W + (size_t)j * stride,
                        W + (size_t)(j + 1) * stride, mx + (size_t)(j - 1) * stride, mx + (size_t)j * stride,
@@ -466,6 +475,17 @@ bool plan_has_fixed(const Plan& p) {
 }
 
 }  // namespace
+
+void scan_segments(const Plan& plan, std::vector<int>& first, std::vector<int>& length) {
+  int h = 0, t = 0;
+  small_runs(plan, h, t);
+  const int cuts[4] = {0, h, std::max(h, t), plan.n};
+  for (int c = 0; c < 3; ++c)
+    for (const Segment& g : segments_of(plan, cuts[c], cuts[c + 1])) {
+      first.push_back(g.j);
+      length.push_back(g.len);
+    }
+}
 
 int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, ChunkLayout& C, int* S_out) {
   *S_out = 0;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <vector>
 
 #include "plan.hpp"
 
@@ -51,6 +52,8 @@ int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, Ch
 // strings keep the position-by-position launch schedule of one tile.
 constexpr long long kOnChipFew = 32, kOnChipMany = 128;
 bool scan_on_chip(const Plan& plan, int precision, long long batch);
+// The passes of a streamed sweep: first position and number of positions of each.
+void scan_segments(const Plan& plan, std::vector<int>& first, std::vector<int>& length);
 // Kernel launches scan_run queues for `batch` items with that workspace.
 int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, size_t ws_bytes, long long* out);
 
@@ -79,6 +82,12 @@ cudaError_t launch_pair_gram_c128(int VE, dim3 grid, cudaStream_t s, const void*
 cudaError_t launch_pair_gram_f32(int VE, dim3 grid, cudaStream_t s, const void* Ein, const DevPair& P,
                                  const unsigned long long* tables, const double4* WA, const unsigned long long* mp,
                                  int lbt, double* partial);
+// A run of positions (P.j ..) over one batch tile (scan_block.cu): weights of position P.j
+// at W, `stride` strings between positions, maxima of the input table at mp and of position
+// P.j at mrow.
+cudaError_t launch_block(int precision, int device, cudaStream_t s, const void* Ein, void* Eout, const DevBlock& P,
+                         const unsigned long long* tables, const double4* W, const unsigned long long* mp,
+                         unsigned long long* mrow, int stride, int lbt);
 // One fused pair (positions P.j, P.j + 1) over one batch tile.
 cudaError_t scan_launch_pair(int precision, int Bt, int device, const DevPair& P, const void* Ein, void* Eout,
                              const unsigned long long* tables, const double4* WA, const double4* WB,

@@ -90,6 +90,17 @@ class ScanPlan:
         _lib.check(L.rgs_plan_pairs(self._h, ctypes.byref(cnt), _lib.ptr(out, ctypes.c_int32)))
         return out[:cnt.value].tolist()
 
+    @property
+    def segments(self):
+        """Passes of a streamed sweep as (first position, positions): one position, a fused
+        pair, or a run whose interior tables stay on chip."""
+        L = _lib.lib()
+        cnt = ctypes.c_int32()
+        first, length = np.zeros(self.n, dtype=np.int32), np.zeros(self.n, dtype=np.int32)
+        _lib.check(L.rgs_plan_segments(self._h, ctypes.byref(cnt), _lib.ptr(first, ctypes.c_int32),
+                                       _lib.ptr(length, ctypes.c_int32)))
+        return list(zip(first[:cnt.value].tolist(), length[:cnt.value].tolist()))
+
     def pair_info(self, k):
         """The k-th fused pair's record (``rgs_pair_info``)."""
         info = _lib.PairInfo()

@@ -1,0 +1,60 @@
+"""Runs of positions (one pass, interior tables in shared memory) against the
+position-by-position sweep.
+
+Plans of rank 18 to 20 whose runs cover every step code the generator gives.  Both sweeps
+round every entry to the storage type and differ in the power-of-two scales and in fused
+multiply-add order nowhere, so amplitudes agree to the storage rounding of renormalised
+tables: the repository's tolerances for fused against unfused sweeps (1e-4 float32
+arithmetic, 1e-5 complex64, 1e-13 complex128 times n positions).  Tile results are bitwise
+equal.  Contraction vectors of size 1e-9 and 1e9 run through the interior scales.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"c64": 1e-5, "c64f32": 1e-4, "c128": 1e-11}
+
+
+def _plans(pkg, count, seed):
+    rng = np.random.default_rng(seed)
+    out, s = [], 0
+    while len(out) < count:
+        s += 1
+        n = 2 * int(rng.integers(17, 28))
+        g = [pkg.instances.regular3, pkg.instances.erdos_renyi, pkg.instances.degree_at_most3][s % 3](n, rng)
+        order = rng.permutation(n).tolist()
+        e = pkg.edges_from_graph(g)
+        if 18 <= max(pkg.rank_profile(n, e, order)) <= 20:
+            out.append((n, pkg.instances.haar_su2(n, rng), pkg.ScanPlan(n, e, order),
+                        pkg.ScanPlan(n, e, order, fuse=False)))
+    return out
+
+
+@pytest.mark.parametrize("precision", ["c64", "c64f32", "c128"])
+def test_runs_match_position_by_position(pkg, precision):
+    import torch
+    rng = np.random.default_rng(2)
+    for n, u, plan, single in _plans(pkg, 4, 11):
+        assert max(k for _, k in plan.segments) > 2 and all(k == 1 for _, k in single.segments)
+        bits = pkg.instances.uniform_bits(24, n, rng)
+        fvec = rng.normal(size=(24, n, 2)) + 1j * rng.normal(size=(24, n, 2))
+        fvec *= 10.0 ** rng.choice([-9, 0, 0, 9], size=(24, n, 1))
+        ref = pkg.ScanEngine(single, u, precision=precision, batch_tile=8)
+        rv, rl = ref.sweep_bits(bits)
+        fv, fl = ref.sweep_fvec(fvec)
+        del ref
+        outs = []
+        for tile in (1, 2, 8, pkg.max_batch_tile(precision)):
+            eng = pkg.ScanEngine(plan, u, precision=precision, batch_tile=tile)
+            v, l = eng.sweep_bits(bits)
+            amp, refamp = v * np.exp(l - 0.35 * n), rv * np.exp(rl - 0.35 * n)
+            assert np.max(np.abs(np.abs(amp / refamp) ** 2 - 1)) < TOL[precision], tile
+            w, m = eng.sweep_fvec(fvec)
+            assert np.max(np.abs(np.abs(w / fv) ** 2 * np.exp(2 * (m - fl)) - 1)) < TOL[precision], tile
+            outs.append((v, l, w, m))
+            del eng
+        for o in outs[1:]:
+            assert all(np.array_equal(x, y) for x, y in zip(o, outs[0]))
+        torch.cuda.empty_cache()
+
