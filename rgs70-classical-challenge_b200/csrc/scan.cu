@@ -506,6 +506,18 @@ bool scan_on_chip(const Plan& plan, int precision, long long batch) {
   return precision != RGS_PREC_C128 || plan.rmax <= 10 || batch <= 1024;
 }
 
+// Tile of the last batch % Bt strings where a smaller one holds them, else 0: a tile costs
+// its full width whatever it holds, so 11 strings in tiles of 8 run as 8 + 4, not 8 + 8
+// (results do not depend on the tile).  Plans of small tables keep one tile size, as their
+// launches, not their bytes, cost.
+int remainder_tile(const Plan& plan, long long batch, int Bt) {
+  const long long rem = batch % Bt;
+  if (rem == 0 || plan.rmax <= kSmallRank) return 0;
+  int t = 1;
+  while (t < rem) t *= 2;
+  return t < Bt ? t : 0;
+}
+
 int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, size_t ws_bytes, long long* out) {
   if (batch < 0) return fail(RGS_ERR_ARG, "batch must be >= 0");
   ScanLayout L;
@@ -516,6 +528,14 @@ int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, 
   if ((rc = scan_pick_chunk(plan, Bt, precision, ws_bytes, C, &S))) return rc;
   const long long n = plan.n;
   long long total = 0;
+  if (const int last = remainder_tile(plan, batch, Bt); last && !scan_on_chip(plan, precision, batch)) {
+    const long long rem = batch % Bt;
+    long long a = 0, b = 0;
+    if (batch > rem && (rc = scan_launch_count(plan, batch - rem, Bt, precision, ws_bytes, &a))) return rc;
+    if ((rc = scan_launch_count(plan, rem, last, precision, ws_bytes, &b))) return rc;
+    *out = a + b;
+    return RGS_OK;
+  }
   if (scan_on_chip(plan, precision, batch)) {
     total = batch ? 1 : 0;
   } else if (S < 2) {
@@ -641,6 +661,19 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
   if (scan_on_chip(plan, precision, batch))
     return scan_run_on_chip(plan, U, bits, fvec, batch, precision, out_value, out_logscale, workspace, ws_bytes, Bt,
                             stream, stats);
+  if (const int last = remainder_tile(plan, batch, Bt)) {
+    const long long rem = batch % Bt, full = batch - rem;
+    const size_t vsize = 2 * (precision == RGS_PREC_C128 ? sizeof(double) : sizeof(float));
+    ScanStats a, b;
+    if (full && (rc = scan_run(plan, U, bits, fvec, full, precision, out_value, out_logscale, workspace, ws_bytes, Bt,
+                               stream, &a)))
+      return rc;
+    rc = scan_run(plan, U, bits ? bits + 2 * full : nullptr, fvec ? fvec + (size_t)full * plan.n * 4 : nullptr, rem,
+                  precision, (char*)out_value + (size_t)full * vsize, out_logscale + full, workspace, ws_bytes, last,
+                  stream, &b);
+    if (stats) stats->launches = a.launches + b.launches;
+    return rc;
+  }
   if (S < 2)
     return scan_run_tiles(plan, U, bits, fvec, batch, precision, out_value, out_logscale, workspace, ws_bytes, Bt,
                           stream, stats);

@@ -1,5 +1,5 @@
 """Runs of positions (one pass, interior tables in shared memory) against the
-position-by-position sweep.
+position-by-position sweep, and remainder tiles.
 
 Plans of rank 18 to 20 whose runs cover every step code the generator gives.  Both sweeps
 round every entry to the storage type and differ in the power-of-two scales and in fused
@@ -58,3 +58,15 @@ def test_runs_match_position_by_position(pkg, precision):
             assert all(np.array_equal(x, y) for x, y in zip(o, outs[0]))
         torch.cuda.empty_cache()
 
+
+def test_remainder_tile(pkg):
+    """A batch's last strings run in the smallest tile that holds them: same results, and the
+    launches that the launch count says."""
+    n, u, plan, _ = _plans(pkg, 1, 5)[0]
+    bits = pkg.instances.uniform_bits(11, n, np.random.default_rng(1))
+    a = pkg.ScanEngine(plan, u, precision="c64f32", batch_tile=8)
+    b = pkg.ScanEngine(plan, u, precision="c64f32", batch_tile=1)
+    (va, la), (vb, lb) = a.sweep_bits(bits), b.sweep_bits(bits)
+    assert np.array_equal(va, vb) and np.array_equal(la, lb)
+    c = pkg.ScanEngine(plan, u, precision="c64f32", batch_tile=4)
+    assert a.launch_count(11) == a.launch_count(8) + c.launch_count(3)
