@@ -406,7 +406,6 @@ bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned
   }
   auto cmask = [&](int i) { return one_at(p.steps[j + i].r_in) - 1; };
   std::vector<Subspace> D(k + 1);
-  const int limit = std::max(kBlockDim, kBlockEnds);
   for (bool changed = true; changed;) {
     changed = false;
     for (int i = 0; i < k; ++i) {
@@ -421,7 +420,7 @@ bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned
         changed |= D[i].add(apply_cols(st.lcols, D[i + 1].basis[b]) & cmask(i));
     }
     for (auto& d : D)
-      if (d.dim() > limit) return false;
+      if (d.dim() > kBlockEnds) return false;
   }
   DevBlock d{};
   d.j = j;
@@ -430,16 +429,33 @@ bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned
   d.r_out = p.steps[j + k - 1].r_out;
   d.din = D[0].dim();
   d.dout = D[k].dim();
+  // Stages, from the right: a growing position joins the next one unless its pair offset
+  // lies in the next one's kernel (or the two are the whole run: the pair kernel's case).
+  auto growing = [&](int i) { return p.dev[j + i].mode == MODE_PAIR && p.dev[j + i].ncombos == 1; };
+  std::vector<int> stage_of(k + 1, -1);  // 1: a fused stage starts here, 0: a single one
+  for (int i = k - 1; i >= 0; --i) {
+    bool join = k > 2 && i > 0 && growing(i - 1);
+    if (join) {
+      Subspace ker;
+      for (u128 v : p.steps[j + i].kernel) ker.add(v & cmask(i));
+      join = ker.add(p.steps[j + i - 1].ycol);
+    }
+    if (join) --i;
+    stage_of[i] = join ? 1 : 0;
+  }
   d.dmax = 0;
-  for (int i = 1; i < k; ++i) d.dmax = std::max(d.dmax, D[i].dim());
-  if (d.din > kBlockEnds || d.dout > kBlockEnds || d.dmax > kBlockDim) return false;
+  for (int i = 0; i <= k; ++i) {
+    if (D[i].dim() > kBlockEnds) return false;
+    if (i > 0 && i < k && stage_of[i] >= 0) d.dmax = std::max(d.dmax, D[i].dim());
+  }
+  if (d.dmax > kBlockDim) return false;
   d.lg = d.r_out - d.dout;
   if (!words_out) return true;  // feasible; the tables are built for chosen runs only
   std::vector<unsigned long long>& words = *words_out;
   auto parity = [](u128 x) {
     return (__builtin_popcountll((uint64_t)x) + __builtin_popcountll((uint64_t)(x >> 64))) & 1;
   };
-  // Slots of the interior levels: linear images of the local basis vectors.
+  // Slots of the levels that have them: linear images of the local basis vectors.
   std::vector<std::vector<unsigned>> slot(k + 1);
   auto slot_of = [&](int i, unsigned c) {
     unsigned s = 0;
@@ -447,76 +463,125 @@ bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned
       if ((c >> b) & 1) s ^= slot[i][b];
     return s;
   };
+  for (int i = 0; i < k; ++i)
+    if (p.dev[j + i].mode == MODE_MERGE) d.merges |= 1u << i;
   std::vector<unsigned long long> prog;
-  for (int i = 0; i < k; ++i) {
-    const PlanStep& st = p.steps[j + i];
-    const DevStep& ds = p.dev[j + i];
-    const bool pair = ds.mode == MODE_PAIR;
-    unsigned tloc = 0;
-    if (pair && !D[i + 1].coords(st.ycol, tloc)) return false;
-    int pivot = -1;  // row operations of a pair: the local rows without this coordinate
-    if (pair)
-      for (int b = 0; b < D[i + 1].dim(); ++b)
-        if ((tloc >> b) & 1) pivot = b;
-    // Slots of level i + 1.
-    if (i == 0) {
-      for (int b = 0; b < D[1].dim(); ++b) slot[1].push_back(1u << b);
-    } else if (i + 1 < k) {
-      unsigned tslot = 0;  // slot offset of a pair's second output
-      if (pair) {
-        for (u128 v : st.kernel) {
-          unsigned c = 0;
-          if (!tslot && (v & cmask(i)) && D[i].coords(v & cmask(i), c)) tslot = slot_of(i, c);
-        }
-        if (!tslot) {  // growth: the lowest slot bit outside the level's span
-          Subspace span;
-          for (unsigned s : slot[i]) span.add(s);
-          for (int b = 0; b < kBlockDim && !tslot; ++b) {
+  for (int i = 0; i < k;) {
+    const bool fused = stage_of[i] == 1;
+    const int ib = fused ? i + 1 : i, o = ib + 1;  // B's position, output level
+    const PlanStep &sa = p.steps[j + i], &sb = p.steps[j + ib];
+    const DevStep& db = p.dev[j + ib];
+    const bool pair = db.mode == MODE_PAIR, last = o == k;
+    // Input row (level i) of a row of level ib, and A's y bit there.
+    auto input_of = [&](u128 row) { return fused ? apply_cols(sa.lcols, row) & cmask(i) : row; };
+    unsigned tloc = 0, vloc = 0;
+    if (pair && !D[o].coords(sb.ycol, tloc)) return false;
+    if (fused && !D[o].coords(apply_cols(sb.mcols, sa.ycol), vloc)) return false;
+    // Row operations: local output rows without the pivot coordinates of t and v.
+    auto top = [](unsigned x) { return 31 - __builtin_clz(x); };
+    const int pt = pair ? top(tloc) : -1;
+    unsigned vred = vloc, tred = tloc;
+    bool v_has_t = false, t_has_v = false;
+    if (fused && pair && ((vloc >> pt) & 1)) {
+      vred ^= tloc;
+      v_has_t = true;
+    }
+    if (fused && !vred) return false;
+    const int pv = fused ? top(vred) : -1;
+    if (fused && pair && ((tloc >> pv) & 1)) {
+      tred ^= vred;
+      t_has_v = true;
+    }
+    // Slots of the output level.
+    if (!last) {
+      if (i == 0) {
+        for (int b = 0; b < D[o].dim(); ++b) slot[o].push_back(1u << b);
+      } else {
+        Subspace span;
+        for (unsigned s : slot[i]) span.add(s);
+        auto fresh = [&]() -> unsigned {  // a slot bit outside the level's span
+          for (int b = 0; b < kBlockDim; ++b) {
             Subspace t = span;
-            if (t.add(one_at(b))) tslot = 1u << b;
+            if (t.add(one_at(b))) {
+              span = t;
+              return 1u << b;
+            }
           }
-          if (!tslot) return false;
+          return 0u;
+        };
+        // Offsets between the inputs of one operation: images of B's kernel.
+        std::vector<unsigned> offs;
+        Subspace seen;
+        for (u128 v : sb.kernel) {
+          unsigned c = 0;
+          const u128 in = input_of(v & cmask(ib));
+          if (!in || !D[i].coords(in, c)) continue;
+          if (seen.add(slot_of(i, c))) offs.push_back(slot_of(i, c));
         }
-      }
-      slot[i + 1].assign(D[i + 1].dim(), 0);
-      for (int b = 0; b < D[i + 1].dim(); ++b) {
-        if (b == pivot) continue;
-        unsigned c = 0;
-        if (!D[i].coords(apply_cols(st.lcols, D[i + 1].at(1u << b)) & cmask(i), c)) return false;
-        slot[i + 1][b] = slot_of(i, c);
-      }
-      if (pair) {
-        // t = pivot vector + others of tloc: the pivot's slot follows from t's.
-        unsigned s = tslot;
-        for (int b = 0; b < D[i + 1].dim(); ++b)
-          if (b != pivot && ((tloc >> b) & 1)) s ^= slot[i + 1][b];
-        slot[i + 1][pivot] = s;
+        size_t next = 0;
+        auto take = [&]() { return next < offs.size() ? offs[next++] : fresh(); };
+        const unsigned st = pair ? take() : 0u, sv = fused ? take() : 0u;
+        if ((pair && !st) || (fused && !sv)) return false;
+        const unsigned s_vred = sv ^ (v_has_t ? st : 0u), s_tred = st ^ (t_has_v ? s_vred : 0u);
+        std::vector<unsigned> base(D[o].dim(), 0);
+        for (int b = 0; b < D[o].dim(); ++b) {
+          if (b == pt || b == pv) continue;
+          unsigned c = 0;
+          if (!D[i].coords(input_of(apply_cols(sb.lcols, D[o].at(1u << b)) & cmask(ib)), c)) return false;
+          base[b] = slot_of(i, c);
+        }
+        slot[o].assign(D[o].dim(), 0);
+        for (int b = 0; b < D[o].dim(); ++b) {
+          unsigned c = 1u << b, s = 0;
+          if (pair && ((c >> pt) & 1)) {
+            c ^= tred;
+            s ^= s_tred;
+          }
+          if (fused && ((c >> pv) & 1)) {
+            c ^= vred;
+            s ^= s_vred;
+          }
+          for (int q = 0; q < D[o].dim(); ++q)
+            if ((c >> q) & 1) s ^= base[q];
+          slot[o][b] = s;
+        }
       }
     }
-    const bool last = i + 1 == k;
-    auto place = [&](unsigned c) { return last ? c : slot_of(i + 1, c); };
-    d.code[i] = pair ? (ds.ncombos == 1 ? RC_P1
-                                        : (ds.ncombos == 2 ? (ds.ng0 == 2 ? RC_P2F : RC_P2H)
-                                                           : (ds.ng0 == 4 ? RC_P4F : RC_P4H)))
-                     : (ds.ncombos == 1 ? RC_M1 : RC_M2);
-    d.first[i] = (int)prog.size();
-    d.pair[i] = pair ? (int)place(tloc) : 0;
-    d.rows[i] = 0;
-    for (unsigned c = 0; c < (1u << D[i + 1].dim()); ++c) {
-      if (pair && ((c >> pivot) & 1)) continue;
-      const u128 l0 = apply_cols(st.lcols, D[i + 1].at(c));
-      const unsigned y0 = pair ? (unsigned)bit_of(l0, st.r_in) : 0u;
+    auto place = [&](unsigned c) { return last ? c : slot_of(o, c); };
+    const int sg = d.stages++;
+    d.step[sg] = i;
+    d.fused[sg] = fused ? 1 : 0;
+    d.code[sg] = pair ? (db.ncombos == 1 ? RC_P1
+                                         : (db.ncombos == 2 ? (db.ng0 == 2 ? RC_P2F : RC_P2H)
+                                                            : (db.ng0 == 4 ? RC_P4F : RC_P4H)))
+                      : (db.ncombos == 1 ? RC_M1 : RC_M2);
+    d.first[sg] = (int)prog.size();
+    d.pair[sg] = pair ? (int)place(tloc) : 0;
+    d.twin[sg] = fused ? (int)place(vloc) : 0;
+    d.twin_sign[sg] = fused ? parity(sa.ycol & sb.beta) : 0;
+    for (unsigned c = 0; c < (1u << D[o].dim()); ++c) {
+      if ((pair && ((c >> pt) & 1)) || (fused && ((c >> pv) & 1))) continue;
+      const u128 l0 = apply_cols(sb.lcols, D[o].at(c));
+      const unsigned y0 = pair ? (unsigned)bit_of(l0, sb.r_in) : 0u;
       unsigned long long w = (unsigned long long)place(y0 ? c ^ tloc : c) << 32;
-      for (int q = 0; q < ds.ncombos; ++q) {
-        const u128 cc = (l0 ^ (u128)ds.combos[q]) & cmask(i);
-        unsigned in = 0;
-        if (!D[i].coords(cc, in)) return false;
-        w |= (unsigned long long)(i == 0 ? in : slot_of(i, in)) << (8 * q);
-        w |= (unsigned long long)parity(cc & st.beta) << (40 + q);
+      for (int q = 0; q < db.ncombos; ++q) {
+        const u128 row = (l0 ^ (u128)db.combos[q]) & cmask(ib);
+        w |= (unsigned long long)parity(row & sb.beta) << (40 + q);
+        u128 in = row;
+        if (fused) {
+          const u128 la = apply_cols(sa.lcols, row);
+          in = la & cmask(i);
+          w |= (unsigned long long)parity(in & sa.beta) << (44 + q);
+          w |= (unsigned long long)bit_of(la, sa.r_in) << (48 + q);
+        }
+        unsigned loc = 0;
+        if (!D[i].coords(in, loc)) return false;
+        w |= (unsigned long long)(i == 0 ? loc : slot_of(i, loc)) << (8 * q);
       }
       prog.push_back(w);
-      ++d.rows[i];
+      ++d.rows[sg];
     }
+    i = o;
   }
   d.words = (int)prog.size();
   // Group maps of every group-index bit, then byte tables.

@@ -119,33 +119,45 @@ struct DevPair {
 // A run of k consecutive free positions j .. j + k - 1 as one pass (scan_block_kernel): the
 // rows of every table of the run fall into groups, cosets of subspaces D_0 (input) .. D_k
 // (output) closed under the run's gathers, so that the rows of one group at one level
-// need only the group's rows of the level before.  A thread carries one string's rows of
-// a group through all k positions in its own shared-memory column.
+// need only the group's rows of the level before.  A thread carries its strings' rows of a
+// group through all k positions in its own shared-memory column.
 // Level i of group g is x_i(g) + D_i, with x_k(g) = g with zeros deposited at the pivots of
 // D_k and x_i the c part of L x_{i+1}; y_i is its y bit and s_i = parity(x_i & beta).  Local
 // rows are coordinates in D_i; the local gathers, signs and destinations do not depend on
 // g except through y_i (swaps a pair's outputs) and s_i (flips every sign).
-// Interior levels live in place: an output row takes the slot of one of its inputs (a
-// growing position adds a slot bit), so a column has 2^dmax slots.
+// A stage is one position, or a growing position A (one combo, two outputs) with the next
+// position B: B's gathers form A's outputs on the way, so the level between them needs no
+// slots.  The other interior levels live in place: an output row takes the slot of one of
+// its inputs (a stage that grows adds slot bits), so a column has 2^dmax slots.
 constexpr int kBlockLen = 6;      // positions per run
-constexpr int kBlockDim = 5;      // dimension of interior levels (32 slots per column)
-constexpr int kBlockEnds = 6;     // dimension of D_0 and D_k
+// Dimension of interior levels with slots (16 per column).  32 slots halve the warps per
+// SM for a few longer runs: 12.2 against 11.6 ms (float32 arithmetic, 4096 strings of the n =
+// 40, rank 20 instance), 22.5 against 21.0 (complex128, 5000), 4.85 against 5.04 (rank 26).
+constexpr int kBlockDim = 4;
+constexpr int kBlockEnds = 6;     // dimension of D_0, D_k and of levels without slots
 constexpr int kBlockRank = 18;    // runs are formed in plans of at least this rank
 struct DevBlock {
   int j, k;
   int r_in, r_out;
   int lg, nbytes;                 // log2 groups; byte tables of the group index
   int din, dout, dmax;
-  int code[kBlockLen];            // ResCode of each position
+  int stages;
+  int step[kBlockLen];            // first position of each stage (relative to j)
+  int fused[kBlockLen];           // the stage is (A, B)
+  int code[kBlockLen];            // ResCode of the stage's (last) position
   int rows[kBlockLen];            // row operations per group
   int first[kBlockLen];           // first program word
   int pair[kBlockLen];            // offset of a pair's second output (slot or local row)
+  int twin[kBlockLen];            // fused: offset of the outputs of the partner gathers
+  int twin_sign[kBlockLen];       // fused: parity(t_A & beta_B)
+  unsigned merges;                // bit i: position j + i is a merge (weights f(0) +- f(1))
   int words;                      // program words
   unsigned long long tab_off;     // u64 index: per (byte, value) the pair (x_0 | x_k << 32,
                                   // y_i at bit 2 i and s_i at bit 2 i + 1), 16-byte aligned
-  // Program word of a row operation: bits 8 c .. 8 c + 5 the slot (first position: local
-  // input row) of combo c, bits 32..37 the slot (last position: local output row) of the
-  // first output for y_i = 0, bit 40 + c the local sign of combo c.
+  // Program word of a row operation: bits 8 c .. 8 c + 5 the slot (first stage: local
+  // input row) of combo c, bits 32..37 the slot (last stage: local output row) of the
+  // first output for y = 0, bit 40 + c the local sign of combo c; fused: bits 44 + c and
+  // 48 + c the local sign and y bit of A at combo c's row.
   unsigned long long prog_off;
   unsigned long long lin_off;     // u32 tables: 2^din input rows, then 2^dout output rows
 };

@@ -10,12 +10,12 @@ cudaError_t launch_block(int precision, int device, cudaStream_t s, const void* 
                          const u64* tables, const double4* W, const u64* mp, u64* mrow, int stride, int lbt) {
   const int sms = sm_count(device);
   if (precision == RGS_PREC_C128)
-    return launch_block_as<double, double, 1, 6>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
+    return launch_block_as<double, double, 1, 8>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
   if (precision == RGS_PREC_C64)
-    return launch_block_as<float, double, 1, 8>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
+    return launch_block_as<float, double, 1, 10>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
   if (lbt >= 1)
-    return launch_block_as<float, float, 2, 6>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
-  return launch_block_as<float, float, 1, 10>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
+    return launch_block_as<float, float, 2, 8>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
+  return launch_block_as<float, float, 1, 14>(device, sms, s, Ein, Eout, P, tables, W, mp, mrow, stride, lbt);
 }
 
 }  // namespace rgs

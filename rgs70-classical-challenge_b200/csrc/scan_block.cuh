@@ -14,13 +14,19 @@
 // 4^e / 4 of the interior tables so that the finalisation's exponents add up.
 //
 // What bounds it: the pair kernels moved 2.8M entries per string of the n = 40, rank 20
-// instance at 79% of the copy bandwidth; runs move 1.1M of the same sweep and are bound by
-// the latency of the column accesses at the ten warps per SM that the columns leave room
-// for (issue slots 38% busy, DRAM 21 to 45%).  Hence a row operation reads one 32-byte
-// record with its ready-made slot offsets, rows and signs (shared memory, the same for
-// every thread), eight gathers are in flight per thread, only the last position tracks
-// maxima, and float32 arithmetic carries two strings per thread (packed FMAs, one set of
-// index work for both).
+// instance at 79% of the copy bandwidth; runs move 1.1M and are bound by instruction issue
+// and the latency of column accesses (peak run of that instance, float32 arithmetic: issue
+// slots 50% busy, DRAM 28%; 16 warps per SM, as many as the columns leave room for).  Hence
+//   * a row operation reads one 32-byte record with its ready-made slot offsets, rows and
+//     signs (shared memory, the same for every thread), several gathers are in flight per
+//     thread, only the last stage tracks maxima;
+//   * a growing position and the next one form one stage, so that the level of the peak rank
+//     has no slots: 16 slots per column instead of 32, and half the column traffic (4096
+//     strings 13.8 -> 11.6 ms, 5000 strings in complex128 25.7 -> 21.0 ms);
+//   * float32 arithmetic carries two strings per thread (packed FMAs, one set of index work
+//     for both).
+// Fetching the next group's maps ahead changed nothing (11.6 ms), prefetching its rows into
+// L2 cost 4%.
 #pragma once
 #include <atomic>
 
@@ -30,14 +36,15 @@
 namespace rgs {
 
 // Threads per block.  64: two warps share the row operations, and blocks are small enough
-// to fill an SM's shared memory (4096 strings of the n = 40 instance, float32 arithmetic:
-// 13.8 ms with 64, 15.9 with 128, 18.8 with 32; complex128, 5000 strings: 25.7 / 29.7 / 36.1).
+// to fill an SM's shared memory (with 32 slots per column, 4096 strings of the n = 40
+// instance, float32 arithmetic: 13.8 ms with 64, 15.9 with 128, 18.8 with 32; complex128,
+// 5000 strings: 25.7 / 29.7 / 36.1).
 constexpr int kBlockThreads = 64, kBlockLogThreads = 6;
 
 struct __align__(16) BlockOp {
   unsigned ld[4];   // slot byte offset, or (first position) input row of each combo
   unsigned st;      // slot byte offset, or (last position) output row of the first output
-  unsigned sign;    // local sign of combo c at bit 31 - c
+  unsigned sign;    // bits 31 - c: local sign of combo c; fused: 27 - c: A's sign, 23 - c: A's y
   unsigned pad[2];
 };
 
@@ -152,15 +159,22 @@ struct BlockStep {
   unsigned x0, xk;     // the group's input and output rows
   unsigned swap;       // xor of the first output's place where the group's y is 1
   unsigned pair;       // xor between a pair's two places
-  unsigned flip;       // 0xf0000000 where the group's sign is 1
+  unsigned flip;       // the group's signs (and A's y), xor-ed into BlockOp::sign
+  unsigned twin;       // fused: xor between the two gathers' places
+  unsigned twin_sign;  // fused: 0x80000000 where the twin gather's signs are flipped
 };
 
-// U row operations, their gathers in flight together.
-template <typename L, typename S, int NV, bool PAIR, int NC, int NG0, bool FIRST, bool LAST, int U>
+// U row operations, their gathers in flight together.  FUSED: a growing position A before
+// B: combo c's gathered entry e gives the two rows e f_A(0) and +-e f_A(1) of A's output;
+// the one with the gather's y bit goes to the operation itself, the other to its twin
+// (same kappa pattern, own signs), so both of A's outputs are used as they are formed.
+template <typename L, typename S, int NV, bool FUSED, bool PAIR, int NC, int NG0, bool FIRST, bool LAST, int U>
 __device__ __forceinline__ void block_ops(const BlockOp* __restrict__ ops, const BlockStep& g,
                                           const BlockCoef<typename L::R>& wa, const BlockCoef<typename L::R>& wb,
+                                          const BlockCoef<typename L::R>& pa, const BlockCoef<typename L::R>& pb,
                                           S (&mx)[NV]) {
   typedef typename L::E E;
+  constexpr int NT = FUSED ? 2 : 1;
   E e[U][NC];
   unsigned sign[U], st[U];
 #pragma unroll
@@ -177,57 +191,78 @@ __device__ __forceinline__ void block_ops(const BlockOp* __restrict__ ops, const
   }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    E a{L::zero(), L::zero()}, b{L::zero(), L::zero()};
+    E a[NT], b[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) a[t] = b[t] = E{L::zero(), L::zero()};
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      const E x = e[u][c];
-      const unsigned m = sign[u] << c;
-      if (PAIR) {
-        const typename L::R nr = L::flip(x.re, m), ni = L::flip(x.im, m);
-        if (c < NG0) {
-          block_mad<L>(a, x.re, x.im, wa);
-          block_mad<L>(b, nr, ni, wb);
+      E x[NT];
+      x[0] = e[u][c];
+      if constexpr (FUSED) {
+        E p{L::zero(), L::zero()}, q{L::zero(), L::zero()};
+        block_mad<L>(p, e[u][c].re, e[u][c].im, pa);
+        block_mad<L>(q, L::flip(e[u][c].re, sign[u] << (4 + c)), L::flip(e[u][c].im, sign[u] << (4 + c)), pb);
+        const bool y = (sign[u] << (8 + c)) & 0x80000000u;
+        x[0].re = y ? q.re : p.re;
+        x[0].im = y ? q.im : p.im;
+        x[NT - 1].re = y ? p.re : q.re;
+        x[NT - 1].im = y ? p.im : q.im;
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const unsigned m = (sign[u] << c) ^ (t ? g.twin_sign : 0u);
+        if (PAIR) {
+          const typename L::R nr = L::flip(x[t].re, m), ni = L::flip(x[t].im, m);
+          if (c < NG0) {
+            block_mad<L>(a[t], x[t].re, x[t].im, wa);
+            block_mad<L>(b[t], nr, ni, wb);
+          } else {
+            block_mad<L>(a[t], nr, ni, wb);
+            block_mad<L>(b[t], x[t].re, x[t].im, wa);
+          }
         } else {
-          block_mad<L>(a, nr, ni, wb);
-          block_mad<L>(b, x.re, x.im, wa);
+          block_mad<L>(a[t], x[t].re, x[t].im, (m & 0x80000000u) ? wb : wa);
         }
-      } else {
-        block_mad<L>(a, x.re, x.im, (m & 0x80000000u) ? wb : wa);
       }
     }
-    const unsigned place = st[u] ^ g.swap;
-    if (LAST) {
-      const unsigned row = g.xk ^ place;
-      L::to_row(g.out + (u64)row * g.pitch, a, mx);
-      if (PAIR) L::to_row(g.out + (u64)(row ^ g.pair) * g.pitch, b, mx);
-    } else {
-      L::to_slot(g.col + place, a);
-      if (PAIR) L::to_slot(g.col + (place ^ g.pair), b);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const unsigned place = st[u] ^ g.swap ^ (t ? g.twin : 0u);
+      if (LAST) {
+        const unsigned row = g.xk ^ place;
+        L::to_row(g.out + (u64)row * g.pitch, a[t], mx);
+        if (PAIR) L::to_row(g.out + (u64)(row ^ g.pair) * g.pitch, b[t], mx);
+      } else {
+        L::to_slot(g.col + place, a[t]);
+        if (PAIR) L::to_slot(g.col + (place ^ g.pair), b[t]);
+      }
     }
   }
 }
 
-// A position's row operations (a power of two), U at a time or, below U, one by one.
-template <typename L, typename S, int NV, bool PAIR, int NC, int NG0, bool FIRST, bool LAST>
+// A stage's row operations (a power of two), U at a time or, below U, one by one.
+template <typename L, typename S, int NV, bool FUSED, bool PAIR, int NC, int NG0, bool FIRST, bool LAST>
 __device__ __forceinline__ void block_rows(const BlockOp* __restrict__ ops, int rows, const BlockStep& g,
-                                           const BlockCoef<typename L::R>& wa, const BlockCoef<typename L::R>& wb,
-                                           S (&mx)[NV]) {
-  constexpr int LOADS = 8;
+                                           const BlockWeights<L>& w, const BlockWeights<L>& wp, S (&mx)[NV]) {
+  constexpr int LOADS = FUSED ? 4 : 8;
   constexpr int U = LOADS >= NC ? LOADS / NC : 1;
+  const BlockCoef<typename L::R> wa{w.ar, w.ai, L::neg(w.ai)}, wb{w.br, w.bi, L::neg(w.bi)};
+  const BlockCoef<typename L::R> pa{wp.ar, wp.ai, L::neg(wp.ai)}, pb{wp.br, wp.bi, L::neg(wp.bi)};
   if (U > 1 && rows < U) {
 #pragma unroll 1
-    for (int r = 0; r < rows; ++r) block_ops<L, S, NV, PAIR, NC, NG0, FIRST, LAST, 1>(ops + r, g, wa, wb, mx);
+    for (int r = 0; r < rows; ++r)
+      block_ops<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, 1>(ops + r, g, wa, wb, pa, pb, mx);
     return;
   }
 #pragma unroll 1
-  for (int r = 0; r < rows; r += U) block_ops<L, S, NV, PAIR, NC, NG0, FIRST, LAST, U>(ops + r, g, wa, wb, mx);
+  for (int r = 0; r < rows; r += U)
+    block_ops<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, U>(ops + r, g, wa, wb, pa, pb, mx);
 }
 
-template <typename L, typename S, int NV, bool FIRST, bool LAST>
-__device__ __forceinline__ void block_step(int code, const BlockOp* ops, int rows, const BlockStep& g,
-                                           const BlockWeights<L>& w, S (&mx)[NV]) {
-  const BlockCoef<typename L::R> wa{w.ar, w.ai, L::neg(w.ai)}, wb{w.br, w.bi, L::neg(w.bi)};
-#define RGS_BLOCK_ROWS(PAIR, NC, NG0) block_rows<L, S, NV, PAIR, NC, NG0, FIRST, LAST>(ops, rows, g, wa, wb, mx)
+template <typename L, typename S, int NV, bool FUSED, bool FIRST, bool LAST>
+__device__ __forceinline__ void block_stage(int code, const BlockOp* ops, int rows, const BlockStep& g,
+                                            const BlockWeights<L>& w, const BlockWeights<L>& wp, S (&mx)[NV]) {
+#define RGS_BLOCK_ROWS(PAIR, NC, NG0) block_rows<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST>(ops, rows, g, w, wp, mx)
   switch (code) {
     case RC_P1: RGS_BLOCK_ROWS(true, 1, 1); break;
     case RC_P2H: RGS_BLOCK_ROWS(true, 2, 1); break;
@@ -269,8 +304,8 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
   BlockOp* ops = reinterpret_cast<BlockOp*>(reinterpret_cast<unsigned char*>(wts) + sizeof(BlockWeights<L>) * T * k);
   const unsigned* lin = reinterpret_cast<const unsigned*>(tables + P.lin_off);
 
-  for (int i = 0; i < k; ++i) {
-    const bool first = i == 0, last = i + 1 == k;
+  for (int i = 0; i < P.stages; ++i) {
+    const bool first = i == 0, last = i + 1 == P.stages;
     for (int r = tid; r < P.rows[i]; r += T) {
       const u64 w = tables[P.prog_off + P.first[i] + r];
       BlockOp op;
@@ -281,12 +316,14 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
       }
       const unsigned s = (unsigned)(w >> 32) & 63u;
       op.st = last ? __ldg(lin + (1 << P.din) + s) : s * (unsigned)(T * L::bytes);
-      const unsigned sg = (unsigned)(w >> 40) & 15u;
-      op.sign = ((sg & 1u) << 31) | ((sg & 2u) << 29) | ((sg & 4u) << 27) | ((sg & 8u) << 25);
+      op.sign = __brev((unsigned)(w >> 40) & 0xfffu);
       op.pad[0] = op.pad[1] = 0u;
       ops[P.first[i] + r] = op;
     }
-    // Weights of this thread's strings.
+  }
+  // Weights of this thread's strings.
+  for (int i = 0; i < k; ++i) {
+    const bool first = i == 0;
     double ar[NV], ai[NV], br[NV], bi[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
@@ -306,7 +343,7 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
       }
       const double s = ldexp(1.0, -e);
       ar[v] = f.x * s, ai[v] = f.y * s, br[v] = f.z * s, bi[v] = f.w * s;
-      if (P.code[i] == RC_M1 || P.code[i] == RC_M2) {
+      if ((P.merges >> i) & 1) {
         const double pr = ar[v] + br[v], pi = ai[v] + bi[v], mr = ar[v] - br[v], mi = ai[v] - bi[v];
         ar[v] = pr, ai[v] = pi, br[v] = mr, bi[v] = mi;
       }
@@ -336,21 +373,37 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
     }
     g.x0 = (unsigned)rows;
     g.xk = (unsigned)(rows >> 32);
-    unsigned fl = (unsigned)flags;
+    const unsigned fl = (unsigned)flags;
 #pragma unroll 1
-    for (int i = 0; i < k; ++i, fl >>= 2) {
-      const bool last = i + 1 == k;
-      const BlockWeights<L> w = wts[i * T + tid];
-      g.pair = last ? __ldg(lin + (1 << P.din) + P.pair[i]) : (unsigned)P.pair[i] * (unsigned)(T * L::bytes);
-      g.swap = (fl & 1u) ? g.pair : 0u;
-      g.flip = (fl & 2u) ? 0xf0000000u : 0u;
+    for (int i = 0; i < P.stages; ++i) {
+      const bool last = i + 1 == P.stages, fused = P.fused[i] != 0;
+      const int pos = P.step[i];
+      const unsigned f = fl >> (2 * pos);  // y and sign of the stage's position(s)
+      const unsigned fb = fused ? f >> 2 : f;
+      const unsigned unit = (unsigned)(T * L::bytes);
+      g.pair = last ? __ldg(lin + (1 << P.din) + P.pair[i]) : (unsigned)P.pair[i] * unit;
+      g.swap = (fb & 1u) ? g.pair : 0u;
+      g.flip = (fb & 2u) ? 0xf0000000u : 0u;
       const BlockOp* op = ops + P.first[i];
-      if (i == 0)
-        block_step<L, S, NV, true, false>(P.code[i], op, P.rows[i], g, w, mx);
-      else if (last)
-        block_step<L, S, NV, false, true>(P.code[i], op, P.rows[i], g, w, mx);
-      else
-        block_step<L, S, NV, false, false>(P.code[i], op, P.rows[i], g, w, mx);
+      const BlockWeights<L> w = wts[(fused ? pos + 1 : pos) * T + tid];
+      if (fused) {
+        g.flip |= ((f & 2u) ? 0x0f000000u : 0u) | ((f & 1u) ? 0x00f00000u : 0u);
+        g.twin = last ? __ldg(lin + (1 << P.din) + P.twin[i]) : (unsigned)P.twin[i] * unit;
+        g.twin_sign = (unsigned)P.twin_sign[i] << 31;
+        const BlockWeights<L> wp = wts[pos * T + tid];
+        if (i == 0)
+          block_stage<L, S, NV, true, true, false>(P.code[i], op, P.rows[i], g, w, wp, mx);
+        else if (last)
+          block_stage<L, S, NV, true, false, true>(P.code[i], op, P.rows[i], g, w, wp, mx);
+        else
+          block_stage<L, S, NV, true, false, false>(P.code[i], op, P.rows[i], g, w, wp, mx);
+      } else if (i == 0) {
+        block_stage<L, S, NV, false, true, false>(P.code[i], op, P.rows[i], g, w, w, mx);
+      } else if (last) {
+        block_stage<L, S, NV, false, false, true>(P.code[i], op, P.rows[i], g, w, w, mx);
+      } else {
+        block_stage<L, S, NV, false, false, false>(P.code[i], op, P.rows[i], g, w, w, mx);
+      }
     }
   }
 #pragma unroll
