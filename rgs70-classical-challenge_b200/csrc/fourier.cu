@@ -407,7 +407,10 @@ __device__ void tile_rounds(float2* sm, const PassParams& P, int TB, unsigned ma
 }
 
 // MINB resident blocks per SM: 3 (80 registers, no spills) or 4 (64 registers, a few
-// spilled); the plan's tuned variant picks one (fourier_tune).
+// spilled); the plan's variant picks one.  Up to m = 32 (32-bit offsets) a plan starts with
+// four, which fill one block's barriers with another's loads: 2.42 against 2.65 ms at m =
+// 27, 0.096 against 0.104 at 22, 22.2 against 23.3 at 30, equal below 20; beyond, with three
+// until fourier_tune measures.
 template <int MINB>
 __global__ void __launch_bounds__(256, MINB) fourier_pass_kernel(const __grid_constant__ PassParams P) {
   extern __shared__ float2 sm[];
@@ -1125,57 +1128,90 @@ struct DrawResult {
   int status;
 };
 
-// First position i of v[0..n) with prefix(i) <= target < prefix(i) + v[i] (searchsorted
-// side='right' on the inclusive cumulative sum), found by one 1024-thread block.
-// Each thread sums a contiguous chunk; chunk sums are scanned in shared memory.
+// Inverse CDF over n non-negative values by one 1024-thread block.  chunk_sums: each thread
+// sums a contiguous chunk and the chunk sums are scanned (warps by shuffles, then the warp
+// totals), one pass over the values giving the total and every thread's prefix; block_find:
+// the first index whose inclusive cumulative sum exceeds the target (numpy.searchsorted
+// side='right'), at or past the total the last positive value, -1 without one.  A thread
+// owns the targets from its prefix up to the next thread's; where rounding leaves a target
+// behind the thread's own running sum, its last positive value is taken.
+// The draw runs four of these on one block, so its time is their serial part: scanning
+// 1024 partial sums by one thread, and summing the values once for the total and once more
+// for the search, took 83 us (2^15 tile masses, m = 27).
+struct ChunkSums {
+  double own, pre, total;
+};
 template <class Get>
-__device__ long long block_search(long long n, double target, Get get, double* total_out) {
-  __shared__ double part[1024];
-  __shared__ long long found;
-  const int t = threadIdx.x, nt = blockDim.x;
-  const long long chunk = (n + nt - 1) / nt;
+__device__ ChunkSums chunk_sums(long long n, Get get) {
+  __shared__ double warp_total[32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const long long chunk = (n + blockDim.x - 1) / blockDim.x;
   const long long lo = min(n, (long long)t * chunk), hi = min(n, lo + chunk);
-  double s = 0.0;
-  for (long long i = lo; i < hi; ++i) s += get(i);
-  part[t] = s;
-  if (t == 0) found = -1;
+  ChunkSums c;
+  c.own = 0.0;
+#pragma unroll 8
+  for (long long i = lo; i < hi; ++i) c.own += get(i);
+  double inc = c.own;
+  for (int o = 1; o < 32; o <<= 1) {
+    const double x = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += x;
+  }
+  __syncthreads();  // the previous call's warp totals have been read
+  if (lane == 31) warp_total[warp] = inc;
+  double exc = __shfl_up_sync(0xffffffffu, inc, 1);
+  if (lane == 0) exc = 0.0;
   __syncthreads();
+  const int nw = blockDim.x >> 5;
+  double w = lane < nw ? warp_total[lane] : 0.0, winc = w;
+  for (int o = 1; o < 32; o <<= 1) {
+    const double x = __shfl_up_sync(0xffffffffu, winc, o);
+    if (lane >= o) winc += x;
+  }
+  const double before = __shfl_sync(0xffffffffu, winc, warp ? warp - 1 : 0);
+  c.pre = (warp ? before : 0.0) + exc;
+  c.total = __shfl_sync(0xffffffffu, winc, 31);
+  return c;
+}
+template <class Get>
+__device__ long long block_find(long long n, const ChunkSums& c, double target, Get get) {
+  __shared__ int owner;
+  __shared__ long long found;
+  const int t = threadIdx.x;
   if (t == 0) {
-    double acc = 0.0;
-    for (int k = 0; k < nt; ++k) {
-      const double x = part[k];
-      part[k] = acc;
-      acc += x;
-    }
-    *total_out = acc;
+    owner = -1;
+    found = -1;
   }
   __syncthreads();
-  const double pre = part[t];
-  if (pre <= target && target < pre + s) {
-    double acc = pre;
+  // The last chunk with mass that starts at or before the target (prefixes ascend with the
+  // thread up to rounding); before every such chunk by rounding: the first one with mass.
+  if (c.own > 0.0 && c.pre <= target) atomicMax(&owner, t);
+  __syncthreads();
+  if (owner < 0) {
+    __syncthreads();
+    if (c.own > 0.0) atomicMax(&owner, 1023 - t);
+    __syncthreads();
+    if (t == 0 && owner >= 0) owner = 1023 - owner;
+    __syncthreads();
+  }
+  if (t == owner) {
+    const long long chunk = (n + blockDim.x - 1) / blockDim.x;
+    const long long lo = min(n, (long long)t * chunk), hi = min(n, lo + chunk);
+    double acc = c.pre;
+    long long last = -1;
     for (long long i = lo; i < hi; ++i) {
       const double x = get(i);
+      if (x > 0.0) last = i;
       if (target < acc + x) {
-        found = i;
+        last = i;
         break;
       }
       acc += x;
     }
+    found = last;
   }
   __syncthreads();
-  long long r = found;
+  const long long r = found;
   __syncthreads();
-  if (r < 0) {  // target at/after the total (rounding): last non-zero entry
-    if (t == 0) {
-      for (long long i = n - 1; i >= 0; --i)
-        if (get(i) > 0.0) {
-          found = i;
-          break;
-        }
-    }
-    __syncthreads();
-    r = found;
-  }
   return r;
 }
 
@@ -1184,13 +1220,10 @@ __global__ void __launch_bounds__(1024) fourier_draw_kernel(const double* __rest
                                                             int deferred, const double2* __restrict__ uT,
                                                             double u1, double u2, double u3,
                                                             DrawResult* __restrict__ out) {
-  __shared__ double norm, tile_total;
-  double tot;
-  // First search (target 0) only establishes the total, then the draw itself.
-  block_search(ntiles, 0.0, [&](long long i) { return masses[i]; }, &tot);
-  if (threadIdx.x == 0) norm = tot;
-  __syncthreads();
-  const long long chosen = block_search(ntiles, u1 * norm, [&](long long i) { return masses[i]; }, &tot);
+  auto mass_at = [&](long long i) { return masses[i]; };
+  const ChunkSums tiles = chunk_sums(ntiles, mass_at);
+  const double norm = tiles.total;
+  const long long chosen = block_find(ntiles, tiles, u1 * norm, mass_at);
   if (chosen < 0) {  // no tile with positive mass: report, read nothing
     if (threadIdx.x == 0) {
       DrawResult r{0ull, 0.0, norm, 2};
@@ -1203,11 +1236,8 @@ __global__ void __launch_bounds__(1024) fourier_draw_kernel(const double* __rest
     const float2 x = v[base + (u64)i];
     return (double)x.x * x.x + (double)x.y * x.y;
   };
-  double tt;
-  block_search(1ll << tile_bits, 0.0, p_at, &tt);
-  if (threadIdx.x == 0) tile_total = tt;
-  __syncthreads();
-  const long long within = block_search(1ll << tile_bits, u2 * tile_total, p_at, &tt);
+  const ChunkSums in_tile = chunk_sums(1ll << tile_bits, p_at);
+  const long long within = block_find(1ll << tile_bits, in_tile, u2 * in_tile.total, p_at);
   if (within < 0) {
     if (threadIdx.x == 0) {
       DrawResult r{0ull, 0.0, norm, 2};
@@ -1245,8 +1275,7 @@ __global__ void __launch_bounds__(1024) fourier_draw_kernel(const double* __rest
 // Total of the tile masses of a shard (the same fixed-order reduction as the draw).
 __global__ void __launch_bounds__(1024) shard_mass_kernel(const double* __restrict__ masses, long long ntiles,
                                                           double* __restrict__ out) {
-  double tot;
-  block_search(ntiles, 0.0, [&](long long i) { return masses[i]; }, &tot);
+  const double tot = chunk_sums(ntiles, [&](long long i) { return masses[i]; }).total;
   if (threadIdx.x == 0) *out = tot;
 }
 
@@ -1711,6 +1740,7 @@ std::string fourier_build(int n, const uint8_t* graph, const double* unitaries, 
   auto g = [&](int a, int b) { return graph[(size_t)a * n + b] != 0; };
   p.n = n;
   p.m = m;
+  p.variant = m <= 32 ? 1 : 0;
   p.A.assign(A, A + m);
   p.B.assign(B, B + m);
   p.deferred = deferred;

@@ -25,7 +25,7 @@ struct FourierPlan {
   std::vector<int> A, B;
   bool specialized = false;      // all U_B identical: popcount weight table (init_specialization.py)
   bool deferred = true;          // terminal unitary on bit m-1 applied at draw time
-  int variant = 0;               // pass-kernel launch variant (fourier_tune)
+  int variant = 0;               // pass-kernel launch variant: 0 three, 1 four blocks per SM (fourier_tune)
   int chunks = 0;
   std::vector<u64h> lut_z;       // [chunks][256][2] covariant map + transformed q_B
   std::vector<u64h> lut_a;       // [chunks][256][2] q_A phase (entry[0] = 0)
