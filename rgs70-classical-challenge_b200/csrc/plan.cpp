@@ -133,16 +133,11 @@ void byte_tables(const std::vector<u128>& cols, int nbits, std::vector<u128>& ou
   // scan_plan.py:133-145
   nbytes = std::max(1, (nbits + 7) / 8);
   out.assign((size_t)nbytes * 256, 0);
-  for (int b = 0; b < nbytes; ++b) {
-    for (int value = 0; value < 256; ++value) {
-      u128 acc = 0;
-      for (int t = 0; t < 8; ++t) {
-        int i = 8 * b + t;
-        if (i < nbits && ((value >> t) & 1)) acc ^= cols[i];
-      }
-      out[(size_t)b * 256 + value] = acc;
+  for (int b = 0; b < nbytes; ++b)
+    for (int v = 1; v < 256; ++v) {  // entry of v: that of v without its lowest bit, and the bit's column
+      const int i = 8 * b + __builtin_ctz((unsigned)v);
+      out[(size_t)b * 256 + v] = out[(size_t)b * 256 + (v & (v - 1))] ^ (i < nbits ? cols[i] : (u128)0);
     }
-  }
 }
 
 std::vector<u128> kernel_combos(const std::vector<u128>& kernel) {
@@ -362,26 +357,33 @@ void build_pairs(Plan& p) {
   p.tables.insert(p.tables.end(), mb.begin(), mb.end());
 }
 
-// A subspace as a reduced echelon basis (highest-bit pivots, each pivot in one vector).
+// A small subspace as a reduced echelon basis (highest-bit pivots, each pivot in one vector).
 struct Subspace {
-  std::vector<u128> basis;
-  std::vector<int> piv;
+  static constexpr int kMax = 8;
+  u128 basis[kMax];
+  int piv[kMax];
+  int n = 0;
+  bool full = false;  // a vector beyond kMax was added
+  int dim() const { return n; }
   bool add(u128 v) {
-    for (size_t i = 0; i < basis.size(); ++i)
+    for (int i = 0; i < n; ++i)
       if (bit_of(v, piv[i])) v ^= basis[i];
     if (!v) return false;
+    if (n == kMax) {
+      full = true;
+      return false;
+    }
     const int h = highest_bit(v);
-    for (auto& b : basis)
-      if (bit_of(b, h)) b ^= v;
-    basis.push_back(v);
-    piv.push_back(h);
+    for (int i = 0; i < n; ++i)
+      if (bit_of(basis[i], h)) basis[i] ^= v;
+    basis[n] = v;
+    piv[n++] = h;
     return true;
   }
-  int dim() const { return (int)basis.size(); }
   // Coordinates of v; false when v lies outside.
   bool coords(u128 v, unsigned& c) const {
     c = 0;
-    for (size_t i = 0; i < basis.size(); ++i)
+    for (int i = 0; i < n; ++i)
       if (bit_of(v, piv[i])) {
         c |= 1u << i;
         v ^= basis[i];
@@ -390,38 +392,63 @@ struct Subspace {
   }
   u128 at(unsigned c) const {
     u128 v = 0;
-    for (size_t i = 0; i < basis.size(); ++i)
+    for (int i = 0; i < n; ++i)
       if ((c >> i) & 1) v ^= basis[i];
     return v;
   }
 };
 
-// The record of the run [j, j + k), or false when its closed subspaces are too large.
-// Appends the run's tables (u64 words, offsets relative to the end of p.tables).
-bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned long long>* words_out) {
+// apply_cols over the set bits of a row of at most 64 bits.
+u128 apply_row(const std::vector<u128>& cols, u128 x) {
+  u128 r = 0;
+  for (uint64_t w = (uint64_t)x; w; w &= w - 1) r ^= cols[__builtin_ctzll(w)];
+  return r;
+}
+
+// Closes D[level] over `v` and its images: M of the positions after a level, the c part of L
+// of the positions before it, for levels 0 .. D.size() - 1 of the run from position j.
+// False when a level outgrows kBlockEnds.
+bool close_over(const Plan& p, int j, std::vector<Subspace>& D, int level, u128 v) {
+  std::vector<std::pair<int, u128>> todo{{level, v}};
+  while (!todo.empty()) {
+    const auto [l, x] = todo.back();
+    todo.pop_back();
+    if (!D[l].add(x)) {
+      if (D[l].full) return false;
+      continue;
+    }
+    if (D[l].dim() > kBlockEnds) return false;
+    if (l + 1 < (int)D.size()) todo.push_back({l + 1, apply_row(p.steps[j + l].mcols, x)});
+    if (l > 0) {
+      const PlanStep& st = p.steps[j + l - 1];
+      todo.push_back({l - 1, apply_row(st.lcols, x) & (one_at(st.r_in) - 1)});
+    }
+  }
+  return true;
+}
+
+// Appends position j + i to the closed levels D[0 .. i] of a run: the images of level i, the
+// pair offset, the kernel.
+bool extend_run(const Plan& p, int j, int i, std::vector<Subspace>& D) {
+  const PlanStep& st = p.steps[j + i];
+  if (!st.free || st.r_in > 31 || st.r_out > 31) return false;
+  D.push_back(Subspace());
+  const Subspace before = D[i];
+  for (int b = 0; b < before.dim(); ++b)
+    if (!close_over(p, j, D, i + 1, apply_row(st.mcols, before.basis[b]))) return false;
+  if (st.ycol && !close_over(p, j, D, i + 1, st.ycol)) return false;
+  for (u128 v : st.kernel)
+    if (!close_over(p, j, D, i, v & (one_at(st.r_in) - 1))) return false;
+  return true;
+}
+
+// The record of the run [j, j + k) with closed levels D, or false when they are too large.
+// words_out: appends the run's tables (u64 words, offsets from the start of p.tables); null:
+// feasibility only.
+bool make_block(const Plan& p, int j, int k, const std::vector<Subspace>& D, DevBlock& out,
+                std::vector<unsigned long long>* words_out) {
   if (k < 2 || k > kBlockLen || j < 1 || j + k > p.n) return false;
-  for (int i = 0; i < k; ++i) {
-    const PlanStep& st = p.steps[j + i];
-    if (!st.free || st.r_in > 31 || st.r_out > 31) return false;
-  }
   auto cmask = [&](int i) { return one_at(p.steps[j + i].r_in) - 1; };
-  std::vector<Subspace> D(k + 1);
-  for (bool changed = true; changed;) {
-    changed = false;
-    for (int i = 0; i < k; ++i) {
-      const PlanStep& st = p.steps[j + i];
-      if (st.ycol) changed |= D[i + 1].add(st.ycol);
-      for (size_t b = 0; b < D[i].basis.size(); ++b) changed |= D[i + 1].add(apply_cols(st.mcols, D[i].basis[b]));
-    }
-    for (int i = k - 1; i >= 0; --i) {
-      const PlanStep& st = p.steps[j + i];
-      for (u128 v : st.kernel) changed |= D[i].add(v & cmask(i));
-      for (size_t b = 0; b < D[i + 1].basis.size(); ++b)
-        changed |= D[i].add(apply_cols(st.lcols, D[i + 1].basis[b]) & cmask(i));
-    }
-    for (auto& d : D)
-      if (d.dim() > kBlockEnds) return false;
-  }
   DevBlock d{};
   d.j = j;
   d.k = k;
@@ -588,7 +615,7 @@ bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned
   std::vector<unsigned long long> rows_of(d.lg), flags_of(d.lg);
   int bit = 0;
   for (int pos = 0; pos < d.r_out; ++pos) {
-    if (std::find(D[k].piv.begin(), D[k].piv.end(), pos) != D[k].piv.end()) continue;
+    if (std::find(D[k].piv, D[k].piv + D[k].dim(), pos) != D[k].piv + D[k].dim()) continue;
     u128 x = one_at(pos);
     unsigned long long flags = 0;
     const unsigned long long outrow = (unsigned long long)x;
@@ -606,16 +633,15 @@ bool make_block(const Plan& p, int j, int k, DevBlock& out, std::vector<unsigned
   d.nbytes = (d.lg + 7) / 8;
   if ((p.tables.size() + words.size()) & 1) words.push_back(0ull);
   d.tab_off = p.tables.size() + words.size();
+  const size_t tab = words.size();
+  words.resize(tab + (size_t)d.nbytes * 512, 0ull);
   for (int b = 0; b < d.nbytes; ++b)
-    for (int v = 0; v < 256; ++v) {
-      unsigned long long r = 0, f = 0;
-      for (int q = 0; q < 8 && 8 * b + q < d.lg; ++q)
-        if ((v >> q) & 1) {
-          r ^= rows_of[8 * b + q];
-          f ^= flags_of[8 * b + q];
-        }
-      words.push_back(r);
-      words.push_back(f);
+    for (int v = 1; v < 256; ++v) {
+      const int i = 8 * b + __builtin_ctz((unsigned)v);
+      unsigned long long* e = &words[tab + 2 * ((size_t)b * 256 + v)];
+      const unsigned long long* less = &words[tab + 2 * ((size_t)b * 256 + (v & (v - 1)))];
+      e[0] = less[0] ^ (i < d.lg ? rows_of[i] : 0ull);
+      e[1] = less[1] ^ (i < d.lg ? flags_of[i] : 0ull);
     }
   d.prog_off = p.tables.size() + words.size();
   words.insert(words.end(), prog.begin(), prog.end());
@@ -647,11 +673,13 @@ void build_blocks(Plan& p) {
   const double launch = 4096.0;  // entries that one more launch costs, per string
   for (int j = t - 1; j >= lo; --j) {
     best[j] = HUGE_VAL;
+    std::vector<Subspace> D(1);
+    bool open = true;  // a longer run needs larger subspaces at every level
     for (int k = 1; k <= kBlockLen && j + k <= t; ++k) {
       DevBlock d;
-      if (k > 1 && !make_block(p, j, k, d, nullptr)) {
-        // A longer run needs larger subspaces at every level.
-        if (k > 2) break;
+      open = open && extend_run(p, j, k - 1, D);
+      if (k > 1 && (!open || !make_block(p, j, k, D, d, nullptr))) {
+        if (!open) break;
         continue;
       }
       const double c = std::ldexp(1.0, p.steps[j].r_in) + std::ldexp(1.0, p.steps[j + k - 1].r_out) + launch + best[j + k];
@@ -667,7 +695,10 @@ void build_blocks(Plan& p) {
     // Two positions that the pair kernel covers run there (its rows stay in registers).
     if (take[j] < 2 || (take[j] == 2 && p.pair_at[j] >= 0)) continue;
     DevBlock d;
-    if (!make_block(p, j, take[j], d, &words)) {  // not reached: the run was found feasible
+    std::vector<Subspace> D(1);
+    bool ok = true;
+    for (int i = 0; i < take[j]; ++i) ok = ok && extend_run(p, j, i, D);
+    if (!ok || !make_block(p, j, take[j], D, d, &words)) {  // not reached: the run was found feasible
       p.blocks.clear();
       p.block_at.assign(p.n, -1);
       p.run_len.assign(p.n, 0);
