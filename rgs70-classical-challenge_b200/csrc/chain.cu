@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(256, 2) chain_gram_kernel(const S* __restrict_
   constexpr int U = RowsPerIter<NC, CPL, LoadsInFlight<S, double>::value>::value;
   constexpr int NI = CPL * VE;
   __shared__ double red[8][kChainMaxTile][4];  // per warp, per item: G00, G11, Re G01, Im G01
+  chained_start();
   const int Bt = 1 << lbt;
   const int lC = lbt - (VE == 2 ? 1 : 0);
   const int lL = lC < 5 ? lC : 5;
@@ -212,6 +213,7 @@ __global__ void chain_decide_kernel(const double* __restrict__ partial, int nblo
   // One block per item: threads sum strided block partials, then a fixed shuffle tree
   // per warp and the warps in order (deterministic).
   __shared__ double wsum[kDecideThreads / 32][4];
+  chained_start();
   const int b = blockIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (b >= count) {
@@ -308,8 +310,8 @@ __global__ void chain_zero_kernel(double* x, long long first, int count) {
 template <typename S, int VE, int CPL, int MODE, int NC>
 cudaError_t launch_gram(dim3 grid, cudaStream_t s, const void* Ein, const DevStep& st, const u64* T, double* partial,
                         int lbt, int unit) {
-  chain_gram_kernel<S, VE, MODE, NC, CPL><<<grid, 256, 0, s>>>((const S*)Ein, st, T, partial, lbt, unit);
-  return cudaGetLastError();
+  return launch_chained(chain_gram_kernel<S, VE, MODE, NC, CPL>, grid, dim3(256), 0, s, (const S*)Ein, st, T, partial, lbt,
+                        unit);
 }
 
 // Positions that need the Gram pass: pair mode with two or four combos, merge mode.
@@ -453,10 +455,9 @@ int chain_run(Plan& plan, const double* U, long long count, int mode_given, u64 
                                          j == 0);
         if (e != cudaSuccess) return e;
       }
-      chain_decide_kernel<<<Bt, kDecideThreads, 0, stream>>>(
-          partial, L.mass_blocks, analytic, Bt, cnt, j, st.v, U2, mode_given, bits, first, uniforms, plan.n, seed,
-          W + (size_t)j * Bt, out_logp, out_cond1, status);
-      return cudaGetLastError();
+      return launch_chained(chain_decide_kernel, dim3((unsigned)Bt), dim3(kDecideThreads), 0, stream, partial,
+                            L.mass_blocks, analytic, Bt, cnt, j, st.v, U2, mode_given, bits, first, uniforms, plan.n, seed,
+                            W + (size_t)j * Bt, out_logp, out_cond1, status);
     };
     int seg = 0;
     for (int j = 0; j < plan.n; ++seg) {

@@ -33,6 +33,34 @@ namespace rgs {
 
 typedef unsigned long long u64;
 
+// Start of a kernel that launch_chained starts before its predecessor in the stream has
+// finished: lets its own successor start as early, then waits until the predecessor's
+// grid has completed and its writes are visible.  Nothing before this call may touch
+// global memory.  Without the launch attribute both are no-ops.
+__device__ __forceinline__ void chained_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launch with programmatic stream serialisation: the blocks are placed while the previous
+// kernel of the stream drains, which hides the launch latency of short dependent kernels
+// (a chain-rule tile is some 180 of them, 3 us each of which one is the gap).  Only for
+// kernels that begin with chained_start().
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 template <typename M>
 struct Cx {
   M re, im;

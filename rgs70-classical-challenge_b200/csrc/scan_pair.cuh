@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(256, PairBlocks<S, M>::value)
   // Group maps of the low bits of a group index (see the loop below), per block.
   __shared__ I s_low[256][2];
   __shared__ unsigned char s_lowpar[256];
+  chained_start();
   const int Bt = 1 << lbt;
   const int lC = lbt - (VE == 2 ? 1 : 0);  // log2 chunks per row
   const int lL = lC < 5 ? lC : 5;          // log2 lanes per row

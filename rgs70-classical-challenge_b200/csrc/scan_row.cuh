@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(256, 2) scan_row_kernel(const S* __restrict__ 
   constexpr int U = RowsPerIter<NC, CPLG, LoadsInFlight<S, M>::value>::value;
   constexpr int NI = CPL * VE;             // items owned by a lane
   __shared__ u64 smax[256];
+  chained_start();
   const int Bt = 1 << lbt;
   const int lC = lbt - (VE == 2 ? 1 : 0);  // log2 chunks per row
   const int lL = lC < 5 ? lC : 5;          // log2 lanes per row
