@@ -76,10 +76,8 @@ __device__ __forceinline__ double flip31(double x, unsigned sgn) {
   return __hiloint2double(__double2hiint(x) ^ (int)sgn, __double2loint(x));
 }
 
-// scale_exponent (scan_device.cuh) without the square root: for a maximum m2 = g 2^k, g in
-// [0.5, 1), sqrt(m2) = f 2^e with f in [0.5, 1) and e = ceil(k / 2) (the correctly rounded
-// root of the largest g below 1 stays below 1).  `done` becomes 1 on a zero and 2 on a
-// non-finite maximum, with e = 0 from there on.
+// scale_exponent (scan_device.cuh) in the storage type.  `done` becomes 1 on a zero and 2
+// on a non-finite maximum, with e = 0 from there on.
 __device__ __forceinline__ int half_exponent(float m2, int& done) {
   const unsigned x = __float_as_uint(m2) >> 23;  // m2 >= 0
   int k = (int)x - 126;

@@ -102,16 +102,35 @@ int plan_device_copy(Plan& plan, int device, const Plan::DeviceCopy** out) {
 // ------------------------------------------------------------------------------------------------
 // Weights: W[j][b] = (f_v(0), f_v(1)) of item b at position j, and for plans with fixed
 // vertices the flags y | ov << 1 (the affine syndrome offset of scan_plan.py:167-172).
+// Plans without fixed vertices (F null): one thread per item and position (grid.y).  With
+// them, one thread per item walks the positions, as each may shift the later syndromes.
 __global__ void scan_weights_kernel(const DevVert* __restrict__ verts, int n, const double2* __restrict__ U,
                                     const u64* __restrict__ bits, const double2* __restrict__ fvec,
                                     long long first, int count, int Bt, double4* __restrict__ W,
                                     unsigned char* __restrict__ F) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= Bt) return;
+  if (!F) {
+    const int j = blockIdx.y, v = verts[j].v;
+    double4 w = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (b < count) {
+      const long long item = first + b;
+      const double2* f;
+      if (fvec) {
+        f = fvec + ((size_t)item * n + v) * 2;
+      } else {
+        const u64 word = bits ? bits[2 * item + (v >> 6)] : 0ull;
+        f = U + (v * 2 + (int)((word >> (v & 63)) & 1ull)) * 2;
+      }
+      w = make_double4(f[0].x, f[0].y, f[1].x, f[1].y);
+    }
+    W[(size_t)j * Bt + b] = w;
+    return;
+  }
   if (b >= count) {
     for (int j = 0; j < n; ++j) {
       W[(size_t)j * Bt + b] = make_double4(0.0, 0.0, 0.0, 0.0);
-      if (F) F[(size_t)j * Bt + b] = 0;
+      F[(size_t)j * Bt + b] = 0;
     }
     return;
   }
@@ -147,35 +166,50 @@ __global__ void scan_weights_kernel(const DevVert* __restrict__ verts, int n, co
       }
     }
     W[(size_t)j * Bt + b] = make_double4(f0.x, f0.y, f1.x, f1.y);
-    if (F) F[(size_t)j * Bt + b] = (unsigned char)(y | (ov << 1));
+    F[(size_t)j * Bt + b] = (unsigned char)(y | (ov << 1));
   }
+}
+
+dim3 weights_grid(int n, int items, const unsigned char* F) {
+  return dim3((unsigned)((items + 127) / 128), F ? 1u : (unsigned)n);
 }
 
 // ------------------------------------------------------------------------------------------------
 // Final value and log-scale per item (gpu_kernel.py:126-170): value = E[0], logscale =
 // ln2 * sum_j e_j, with e_0 = 1 and e_j from the maximum after step j-1.  An all-zero
 // table ends the sum as in the reference (value 0); a non-finite maximum yields NaN.
+// The exponent sum of one item: max(j) = maxbuf[j * stride].  Maxima are loaded eight
+// positions at a time (one memory round trip each, instead of one per position).
+template <typename S>
+__device__ __forceinline__ long long exponent_sum(const u64* __restrict__ maxbuf, int n, size_t stride, bool& zero,
+                                                  bool& bad) {
+  constexpr int kAhead = 8;
+  long long esum = 0;
+  double m2prev = 1.0;
+  zero = bad = false;
+  for (int j0 = 0; j0 < n && !zero && !bad; j0 += kAhead) {
+    u64 m[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) m[q] = j0 + q < n ? maxbuf[(size_t)(j0 + q) * stride] : 0ull;
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      if (j0 + q >= n || zero || bad) break;
+      esum += scale_exponent(m2prev);
+      m2prev = max_value<S>(m[q]);
+      bad = !isfinite(m2prev);
+      zero = !bad && !(m2prev > 0.0);
+    }
+  }
+  return esum;
+}
+
 template <typename S>
 __global__ void scan_finalize_kernel(const S* __restrict__ E, const u64* __restrict__ maxbuf, int n, int Bt,
                                      int count, S* __restrict__ out_value, double* __restrict__ out_logscale) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= count) return;
-  long long esum = 0;
-  bool zero = false, bad = false;
-  double m2prev = 1.0;
-  for (int j = 0; j < n; ++j) {
-    esum += scale_exponent(m2prev);
-    const double m2 = max_value<S>(maxbuf[(size_t)j * Bt + b]);
-    if (!isfinite(m2)) {
-      bad = true;
-      break;
-    }
-    if (!(m2 > 0.0)) {
-      zero = true;
-      break;
-    }
-    m2prev = m2;
-  }
+  bool zero, bad;
+  const long long esum = exponent_sum<S>(maxbuf + b, n, (size_t)Bt, zero, bad);
   S re = E[2 * (size_t)b], im = E[2 * (size_t)b + 1];
   if (zero) re = im = (S)0;
   if (bad) re = im = (S)NAN;
@@ -192,22 +226,8 @@ __global__ void scan_finalize_chunk_kernel(const S* __restrict__ E, u64 e_stride
                                            S* __restrict__ out_value, double* __restrict__ out_logscale) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  long long esum = 0;
-  bool zero = false, bad = false;
-  double m2prev = 1.0;
-  for (int j = 0; j < n; ++j) {
-    esum += scale_exponent(m2prev);
-    const double m2 = max_value<S>(maxbuf[(size_t)j * stride + i]);
-    if (!isfinite(m2)) {
-      bad = true;
-      break;
-    }
-    if (!(m2 > 0.0)) {
-      zero = true;
-      break;
-    }
-    m2prev = m2;
-  }
+  bool zero, bad;
+  const long long esum = exponent_sum<S>(maxbuf + i, n, (size_t)stride, zero, bad);
   const u64 e = ((u64)(i >> lbt) * e_stride + (u64)(i & ((1 << lbt) - 1))) * 2;
   S re = E[e], im = E[e + 1];
   if (zero) re = im = (S)0;
@@ -618,7 +638,7 @@ int scan_run_tiles(Plan& plan, const double* U, const u64* bits, const double* f
 
   for (long long first = 0; first < batch; first += Bt) {
     const int count = (int)std::min<long long>(Bt, batch - first);
-    scan_weights_kernel<<<(Bt + 127) / 128, 128, 0, stream>>>((const DevVert*)dc->verts, plan.n, (const double2*)U,
+    scan_weights_kernel<<<weights_grid(plan.n, Bt, F), 128, 0, stream>>>((const DevVert*)dc->verts, plan.n, (const double2*)U,
                                                               bits, (const double2*)fvec, first, count, Bt, W, F);
     RGS_CUDA_TRY(cudaGetLastError());
     RGS_CUDA_TRY(cudaMemsetAsync(maxbuf, 0, (size_t)plan.n * Bt * sizeof(u64), stream));
@@ -702,7 +722,7 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
   for (long long first = 0; first < batch; first += stride) {
     const int count = (int)std::min<long long>(stride, batch - first);
     const int tiles = (count + Bt - 1) / Bt;
-    scan_weights_kernel<<<(stride + 127) / 128, 128, 0, stream>>>((const DevVert*)dc->verts, n, (const double2*)U,
+    scan_weights_kernel<<<weights_grid(n, stride, F), 128, 0, stream>>>((const DevVert*)dc->verts, n, (const double2*)U,
                                                                   bits, (const double2*)fvec, first, count, stride, W,
                                                                   F);
     RGS_CUDA_TRY(cudaGetLastError());
@@ -776,7 +796,7 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
 // ------------------------------------------------------------------------------------------------
 cudaError_t scan_launch_weights(const DevVert* verts, int n, const double* U, const u64* bits, const double* fvec,
                                 long long first, int count, int Bt, void* W, unsigned char* F, cudaStream_t stream) {
-  scan_weights_kernel<<<(Bt + 127) / 128, 128, 0, stream>>>(verts, n, (const double2*)U, bits, (const double2*)fvec,
+  scan_weights_kernel<<<weights_grid(n, Bt, F), 128, 0, stream>>>(verts, n, (const double2*)U, bits, (const double2*)fvec,
                                                             first, count, Bt, (double4*)W, F);
   return cudaGetLastError();
 }

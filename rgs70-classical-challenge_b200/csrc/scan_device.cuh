@@ -155,11 +155,19 @@ __device__ __forceinline__ u64 deposit_zero(u64 i, int pi) {
 
 // Power-of-two scale for the next step from the previous maximum |E|^2, exactly as
 // GPUMixin._sweep (gpu_kernel.py:146-148): m = sqrt(max|E|^2), m = f 2^e with
-// f in [0.5, 1), scale = 2^-e.  Returns e; m2 = 1 for the first step.
+// f in [0.5, 1), scale = 2^-e.  Returns e; m2 = 1 for the first step.  From the exponent
+// alone: for m2 = g 2^k, g in [0.5, 1), e = ceil(k / 2) (the correctly rounded root of the
+// largest g below 1 stays below 1); 0 for zero and non-finite maxima.
 __device__ __forceinline__ int scale_exponent(double m2) {
-  int e = 0;
-  frexp(sqrt(m2), &e);
-  return e;
+  const int x = (__double2hiint(m2) >> 20) & 0x7ff;
+  int k = x - 1022;
+  if (x == 0) {
+    if (!(m2 > 0.0)) return 0;
+    k = ((__double2hiint(m2 * 0x1.0p64) >> 20) & 0x7ff) - 1022 - 64;  // subnormal
+  } else if (x == 0x7ff) {
+    return 0;
+  }
+  return (k + 1) >> 1;
 }
 
 // Mass of one branch of a position from the position's Gram matrix G (chain rule):
