@@ -655,27 +655,17 @@ bool make_block(const Plan& p, int j, int k, const std::vector<Subspace>& D, Dev
   return true;
 }
 
-// Chooses the runs of the middle positions (plans of rank >= kBlockRank): segments of one
-// position, one fused pair or one run, minimising the table entries read and written.
-void build_blocks(Plan& p) {
-  p.blocks.clear();
-  p.block_at.assign(p.n, -1);
-  p.run_len.assign(p.n, 0);
-  if (!p.fuse || !p.exec_ok || p.rmax < kBlockRank || p.rmax > 31) return;
-  for (auto& st : p.steps)
-    if (!st.free) return;
-  int h = 0, t = 0;
-  small_runs(p, h, t);
-  const int lo = std::max(h, 1);
-  if (lo >= t) return;
+// Chooses the segments of positions [lo, hi) -- one position, a fused pair or a run --
+// minimising the table entries read and written plus `launch` entries per segment.
+void choose_runs(Plan& p, int lo, int hi, double launch, std::vector<DevBlock>& blocks, std::vector<int>& block_at,
+                 std::vector<int>& run_len) {
   std::vector<double> best(p.n + 1, 0.0);
   std::vector<int> take(p.n + 1, 1);
-  const double launch = 4096.0;  // entries that one more launch costs, per string
-  for (int j = t - 1; j >= lo; --j) {
+  for (int j = hi - 1; j >= lo; --j) {
     best[j] = HUGE_VAL;
     std::vector<Subspace> D(1);
     bool open = true;  // a longer run needs larger subspaces at every level
-    for (int k = 1; k <= kBlockLen && j + k <= t; ++k) {
+    for (int k = 1; k <= kBlockLen && j + k <= hi; ++k) {
       DevBlock d;
       open = open && extend_run(p, j, k - 1, D);
       if (k > 1 && (!open || !make_block(p, j, k, D, d, nullptr))) {
@@ -690,8 +680,8 @@ void build_blocks(Plan& p) {
     }
   }
   std::vector<unsigned long long> words;
-  for (int j = lo; j < t; j += take[j]) {
-    p.run_len[j] = take[j];
+  for (int j = lo; j < hi; j += take[j]) {
+    run_len[j] = take[j];
     // Two positions that the pair kernel covers run there (its rows stay in registers).
     if (take[j] < 2 || (take[j] == 2 && p.pair_at[j] >= 0)) continue;
     DevBlock d;
@@ -699,15 +689,35 @@ void build_blocks(Plan& p) {
     bool ok = true;
     for (int i = 0; i < take[j]; ++i) ok = ok && extend_run(p, j, i, D);
     if (!ok || !make_block(p, j, take[j], D, d, &words)) {  // not reached: the run was found feasible
-      p.blocks.clear();
-      p.block_at.assign(p.n, -1);
-      p.run_len.assign(p.n, 0);
+      blocks.clear();
+      block_at.assign(p.n, -1);
+      run_len.assign(p.n, 0);
       return;
     }
-    p.block_at[j] = (int)p.blocks.size();
-    p.blocks.push_back(d);
+    block_at[j] = (int)blocks.size();
+    blocks.push_back(d);
   }
   p.tables.insert(p.tables.end(), words.begin(), words.end());
+}
+
+// Runs of the middle positions of large plans (rank >= kBlockRank), and of every position
+// of plans whose tables are just small enough for chunks of tiles (kFlatRank and above).
+void build_blocks(Plan& p) {
+  p.blocks.clear();
+  p.block_at.assign(p.n, -1);
+  p.run_len.assign(p.n, 0);
+  p.flat_blocks.clear();
+  p.flat_at.assign(p.n, -1);
+  p.flat_len.assign(p.n, 0);
+  if (!p.fuse || !p.exec_ok || p.rmax > 31) return;
+  for (auto& st : p.steps)
+    if (!st.free) return;
+  int h = 0, t = 0;
+  small_runs(p, h, t);
+  if (p.rmax >= kBlockRank && std::max(h, 1) < t)
+    choose_runs(p, std::max(h, 1), t, 4096.0, p.blocks, p.block_at, p.run_len);
+  if (p.rmax >= kFlatRank && p.rmax <= kSmallRank && p.n > 1)
+    choose_runs(p, 1, p.n, 256.0, p.flat_blocks, p.flat_at, p.flat_len);
 }
 
 // On-chip step records (plans of rank <= kResMaxRank): see ResStep.

@@ -135,7 +135,8 @@ constexpr int kBlockLen = 6;      // positions per run
 // 40, rank 20 instance), 22.5 against 21.0 (complex128, 5000), 4.85 against 5.04 (rank 26).
 constexpr int kBlockDim = 4;
 constexpr int kBlockEnds = 6;     // dimension of D_0, D_k and of levels without slots
-constexpr int kBlockRank = 18;    // runs are formed in plans of at least this rank
+constexpr int kBlockRank = 18;    // runs are formed in plans of at least this rank,
+constexpr int kFlatRank = 9;      // ... and over all positions from here to kSmallRank
 struct DevBlock {
   int j, k;
   int r_in, r_out;
@@ -187,6 +188,9 @@ struct Plan {
   // fused pair), 0 where no segment starts or outside the middle positions.
   std::vector<DevBlock> blocks;
   std::vector<int> block_at, run_len;
+  // The same over every position but the first (kFlatRank <= rank <= kSmallRank).
+  std::vector<DevBlock> flat_blocks;
+  std::vector<int> flat_at, flat_len;
   bool exec_ok = false;
   std::string exec_reason;
   // Device copies, per device ordinal (created lazily by the executor).

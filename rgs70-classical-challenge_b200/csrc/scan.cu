@@ -448,13 +448,15 @@ namespace {
 struct Segment {
   int j, len, pair, block;
 };
-std::vector<Segment> segments_of(const Plan& plan, int from, int to) {
+std::vector<Segment> segments_of(const Plan& plan, int from, int to, bool flat = false) {
   std::vector<Segment> out;
   for (int j = from; j < to;) {
-    const int run = plan.blocks.empty() ? 0 : plan.run_len[j];  // 0: not planned as runs
+    // 0: not planned as runs
+    const int run = flat ? plan.flat_len[j] : (plan.blocks.empty() ? 0 : plan.run_len[j]);
+    const int block = !run ? -1 : (flat ? plan.flat_at[j] : plan.block_at[j]);
     const int pa = plan.pair_at.empty() ? -1 : plan.pair_at[j];
-    if (run && plan.block_at[j] >= 0) {
-      out.push_back({j, run, -1, plan.block_at[j]});
+    if (block >= 0) {
+      out.push_back({j, run, -1, block});
       j += run;
     } else if (pa >= 0 && j + 1 < to && run != 1) {
       out.push_back({j, 2, pa, -1});
@@ -471,12 +473,12 @@ std::vector<Segment> segments_of(const Plan& plan, int from, int to) {
 // `stride` between positions).
 cudaError_t launch_segment(const Plan& plan, const Segment& g, int precision, int Bt, int device, cudaStream_t s,
                            const void* Ein, void* Eout, const u64* tables, const double4* W,
-                           const unsigned char* F, u64* mx, size_t stride, int tiles, u64 es) {
+                           const unsigned char* F, u64* mx, size_t stride, int tiles, u64 es, bool flat = false) {
   const int j = g.j;
-  if (g.block >= 0)  // middle positions: one tile per launch
-    return launch_block(precision, device, s, Ein, Eout, plan.blocks[g.block], tables, W + (size_t)j * stride,
-                        mx + (size_t)(j - 1) * stride, mx + (size_t)j * stride, (int)stride,
-                        __builtin_ctz((unsigned)Bt));
+  if (g.block >= 0)
+    return launch_block(precision, device, s, Ein, Eout, (flat ? plan.flat_blocks : plan.blocks)[g.block], tables,
+                        W + (size_t)j * stride, mx + (size_t)(j - 1) * stride, mx + (size_t)j * stride, (int)stride,
+                        __builtin_ctz((unsigned)Bt), tiles, es);
   if (g.len == 2)
     return launch_pair(precision, Bt, device, s, Ein, Eout, plan.pairs[g.pair], tables, W + (size_t)j * stride,
                        W + (size_t)(j + 1) * stride, mx + (size_t)(j - 1) * stride, mx + (size_t)j * stride,
@@ -519,10 +521,16 @@ int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, Ch
   return RGS_OK;
 }
 
+bool scan_flat(const Plan& plan, int precision, long long batch) {
+  if (plan.flat_blocks.empty()) return false;
+  const int r = plan.rmax + (precision == RGS_PREC_C128 ? 1 : 0);
+  return r >= 10 && batch >= (r >= 13 ? 512 : 1ll << (23 - r));
+}
+
 bool scan_on_chip(const Plan& plan, int precision, long long batch) {
   if (!plan.fuse || !resident_plan_fits(plan)) return false;
   if (batch > kOnChipFew && batch < kOnChipMany) return false;
-  return precision != RGS_PREC_C128 || plan.rmax <= 10 || batch <= 1024;
+  return !scan_flat(plan, precision, batch);
 }
 
 // Tile of the last batch % Bt strings where a smaller one holds them, else 0: a tile costs
@@ -558,12 +566,14 @@ int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, 
   if (scan_on_chip(plan, precision, batch)) {
     total = batch ? 1 : 0;
   } else if (S < 2) {
-    total = (batch + Bt - 1) / Bt * ((long long)segments_of(plan, 0, (int)n).size() + 2);
+    total = (batch + Bt - 1) / Bt *
+            ((long long)segments_of(plan, 0, (int)n, scan_flat(plan, precision, batch)).size() + 2);
   } else {
     const long long stride = (long long)S * Bt;
-    const long long nh = (long long)segments_of(plan, 0, C.h).size();
+    const bool flat = scan_flat(plan, precision, batch);
+    const long long nh = (long long)segments_of(plan, 0, C.h, flat).size();
     const long long nm = (long long)segments_of(plan, C.h, C.t).size();
-    const long long nt = (long long)segments_of(plan, std::max(C.t, C.h), (int)n).size();
+    const long long nt = (long long)segments_of(plan, std::max(C.t, C.h), (int)n, flat).size();
     for (long long first = 0; first < batch; first += stride) {
       const long long tiles = (std::min(stride, batch - first) + Bt - 1) / Bt;
       total += 1 + nh;
@@ -634,7 +644,8 @@ int scan_run_tiles(Plan& plan, const double* U, const u64* bits, const double* f
   u64* maxbuf = (u64*)(ws + L.off_max);
   const u64* tables = (const u64*)dc->tables;
   long long launches = 0;
-  const std::vector<Segment> segs = segments_of(plan, 0, plan.n);
+  const bool flat = scan_flat(plan, precision, batch);
+  const std::vector<Segment> segs = segments_of(plan, 0, plan.n, flat);
 
   for (long long first = 0; first < batch; first += Bt) {
     const int count = (int)std::min<long long>(Bt, batch - first);
@@ -646,7 +657,7 @@ int scan_run_tiles(Plan& plan, const double* U, const u64* bits, const double* f
     int cur = 0;
     for (const Segment& g : segs) {
       RGS_CUDA_TRY(launch_segment(plan, g, precision, Bt, device, stream, buf[cur], buf[cur ^ 1], tables, W, F,
-                                  maxbuf, (size_t)Bt, 1, 0));
+                                  maxbuf, (size_t)Bt, 1, 0, flat));
       cur ^= 1;
       launches += 1;
     }
@@ -716,8 +727,9 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
   const u64* tables = (const u64*)dc->tables;
   const int lbt = __builtin_ctz((unsigned)Bt);
   long long launches = 0;
-  const std::vector<Segment> head = segments_of(plan, 0, h), mid = segments_of(plan, h, t),
-                             tail = segments_of(plan, std::max(t, h), n);
+  const bool flat = scan_flat(plan, precision, batch);
+  const std::vector<Segment> head = segments_of(plan, 0, h, flat), mid = segments_of(plan, h, t),
+                             tail = segments_of(plan, std::max(t, h), n, flat);
 
   for (long long first = 0; first < batch; first += stride) {
     const int count = (int)std::min<long long>(stride, batch - first);
@@ -732,7 +744,7 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
     // Leading small positions: all tiles of the chunk per launch.
     for (const Segment& g : head) {
       RGS_CUDA_TRY(launch_segment(plan, g, precision, Bt, device, stream, small[cur], small[cur ^ 1], tables, W, F,
-                                  maxbuf, (size_t)stride, tiles, C.e_stride));
+                                  maxbuf, (size_t)stride, tiles, C.e_stride, flat));
       cur ^= 1;
       launches += 1;
     }
@@ -773,7 +785,7 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
     if (t < n || h == n) {
       for (const Segment& g : tail) {
         RGS_CUDA_TRY(launch_segment(plan, g, precision, Bt, device, stream, small[cur], small[cur ^ 1], tables, W,
-                                    F, maxbuf, (size_t)stride, tiles, C.e_stride));
+                                    F, maxbuf, (size_t)stride, tiles, C.e_stride, flat));
         cur ^= 1;
         launches += 1;
       }

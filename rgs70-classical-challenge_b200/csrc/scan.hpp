@@ -43,15 +43,21 @@ int scan_chunk_tiles(int Bt);
 // scan_chunk_tiles(Bt), S >= 2, whose layout fits, with C filled in); 0: tile by tile.
 int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, ChunkLayout& C, int* S);
 // Whether scan_run sweeps `batch` strings of a plan on chip, as one launch (resident.cu),
-// instead of one launch per position: plans of rank <= kResPlanRank with fusion on.
-// Measured, on chip against streamed: one string 31 against 166 us (rank 9, n = 40), 300
-// strings 44 against 266 us (rank 10), 8192 strings 183 against 422 us (rank 10, complex64,
-// float32 arithmetic), 975 against 1210 us (rank 12); complex128 at rank 11: 181 against
-// 295 us for 1000 strings, but 1026 against 836 us for 8192 (three units per SM: too few
-// warps), so large complex128 batches above rank 10 are streamed.  Sweeps of 33 to 127
-// strings keep the position-by-position launch schedule of one tile.
+// instead of one launch per segment: plans of rank <= kResPlanRank with fusion on, below
+// the batches of scan_flat.  Measured, on chip against fused pairs: one string 31 against
+// 166 us (rank 9, n = 40), 300 strings 50 against 207 us (rank 10, complex64, float32
+// arithmetic).  Sweeps of 33 to 127 strings keep the position-by-position launch schedule
+// of one tile.
 constexpr long long kOnChipFew = 32, kOnChipMany = 128;
 bool scan_on_chip(const Plan& plan, int precision, long long batch);
+// Whether such a plan is swept as runs over all its positions, one launch per run and chunk
+// of tiles: from a batch whose tables hold 2^23 complex64 entries (half as many strings
+// per rank), or 512 strings of rank 12 in complex128, whose tables leave an SM one unit on
+// chip.  Measured, on chip / runs: rank 12, float32 arithmetic, 1000 strings 176 / 179 us,
+// 2048 286 / 222, 8192 993 / 446; rank 11, 4096 strings 244 / 206 (n = 56) and 139 / 143 (n
+// = 26); rank 10, 4096 strings 125 / 155, 8192 197 / 186; complex128, rank 12, 300 strings
+// 194 / 161, 1000 419 / 204; rank 9, 4096 strings 119 / 111 and 87 / 93, 8192 192 / 131.
+bool scan_flat(const Plan& plan, int precision, long long batch);
 // The passes of a streamed sweep: first position and number of positions of each.
 void scan_segments(const Plan& plan, std::vector<int>& first, std::vector<int>& length);
 // Kernel launches scan_run queues for `batch` items with that workspace.
@@ -87,7 +93,7 @@ cudaError_t launch_pair_gram_f32(int VE, dim3 grid, cudaStream_t s, const void* 
 // P.j at mrow.
 cudaError_t launch_block(int precision, int device, cudaStream_t s, const void* Ein, void* Eout, const DevBlock& P,
                          const unsigned long long* tables, const double4* W, const unsigned long long* mp,
-                         unsigned long long* mrow, int stride, int lbt);
+                         unsigned long long* mrow, int stride, int lbt, int tiles, unsigned long long es);
 // One fused pair (positions P.j, P.j + 1) over one batch tile.
 cudaError_t scan_launch_pair(int precision, int Bt, int device, const DevPair& P, const void* Ein, void* Eout,
                              const unsigned long long* tables, const double4* WA, const double4* WB,

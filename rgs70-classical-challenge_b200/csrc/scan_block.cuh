@@ -285,12 +285,12 @@ __host__ __device__ constexpr size_t block_smem_bytes(int dmax, int k, int words
 
 // W: weights of position j, `stride` strings between positions; maxprev: maxima of the
 // input table; maxrow: row of position j of the maxima.  blockIdx.x: column slice (tiles
-// wider than the block), then groups.
+// wider than the block), then groups; blockIdx.y: tile, tables e_stride entries apart.
 template <typename S, typename M, int NV, int MINB>
 __global__ void __launch_bounds__(kBlockThreads, MINB)
     scan_block_kernel(const S* __restrict__ Ein, S* __restrict__ Eout, const __grid_constant__ DevBlock P,
                       const u64* __restrict__ tables, const double4* __restrict__ W, const u64* __restrict__ maxprev,
-                      u64* __restrict__ maxrow, int stride, int lbt) {
+                      u64* __restrict__ maxrow, int stride, int lbt, u64 e_stride) {
   typedef BlockLane<S, M, NV> L;
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int T = kBlockThreads, kLT = kBlockLogThreads, kLV = NV == 2 ? 1 : 0;
@@ -303,6 +303,14 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
   BlockWeights<L>* wts = reinterpret_cast<BlockWeights<L>*>(smem + (((size_t)L::bytes << P.dmax) * T));
   BlockOp* ops = reinterpret_cast<BlockOp*>(reinterpret_cast<unsigned char*>(wts) + sizeof(BlockWeights<L>) * T * k);
   const unsigned* lin = reinterpret_cast<const unsigned*>(tables + P.lin_off);
+  if (blockIdx.y) {  // tile y of a chunk of tiles
+    const u64 y = blockIdx.y;
+    Ein += 2 * y * e_stride;
+    Eout += 2 * y * e_stride;
+    W += y << lbt;
+    maxprev += y << lbt;
+    maxrow += y << lbt;
+  }
 
   for (int i = 0; i < P.stages; ++i) {
     const bool first = i == 0, last = i + 1 == P.stages;
@@ -413,7 +421,8 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
 
 template <typename S, typename M, int NV, int MINB>
 cudaError_t launch_block_as(int device, int sms, cudaStream_t s, const void* Ein, void* Eout, const DevBlock& P,
-                            const u64* tables, const double4* W, const u64* mp, u64* mrow, int stride, int lbt) {
+                            const u64* tables, const double4* W, const u64* mp, u64* mrow, int stride, int lbt,
+                            int tiles, u64 es) {
   typedef BlockLane<S, M, NV> L;
   const size_t smem = block_smem_bytes<L>(P.dmax, P.k, P.words);
   static std::atomic<bool> configured[64];  // the attribute is per device; setting it twice is harmless
@@ -429,11 +438,11 @@ cudaError_t launch_block_as(int device, int sms, cudaStream_t s, const void* Ein
   const int lcols = lc < kBlockLogThreads ? lc : kBlockLogThreads, lslices = lc - lcols, lslots = kBlockLogThreads - lcols;
   const u64 units = ((1ull << P.lg) + (1ull << lslots) - 1) >> lslots;  // group sets
   const u64 fit = 227 * 1024 / (smem + 1024);
-  u64 per_slice = ((u64)sms * (fit < MINB ? fit : MINB)) >> lslices;
+  u64 per_slice = (((u64)sms * (fit < MINB ? fit : MINB)) >> lslices) / (u64)tiles;
   if (per_slice < 1) per_slice = 1;
   if (per_slice > units) per_slice = units;
-  scan_block_kernel<S, M, NV, MINB><<<(unsigned)(per_slice << lslices), kBlockThreads, smem, s>>>(
-      (const S*)Ein, (S*)Eout, P, tables, W, mp, mrow, stride, lbt);
+  scan_block_kernel<S, M, NV, MINB><<<dim3((unsigned)(per_slice << lslices), (unsigned)tiles), kBlockThreads, smem, s>>>(
+      (const S*)Ein, (S*)Eout, P, tables, W, mp, mrow, stride, lbt, es);
   return cudaGetLastError();
 }
 

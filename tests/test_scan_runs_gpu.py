@@ -59,6 +59,45 @@ def test_runs_match_position_by_position(pkg, precision):
         torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("precision,rank,count", [("c64f32", 12, 2050), ("c64", 11, 4099), ("c64f32", 10, 8192),
+                                                  ("c128", 9, 8200), ("c128", 12, 513)])
+def test_runs_over_all_positions(pkg, precision, rank, count):
+    """Low-rank plans on batches large enough for runs over every position, at two tiles and
+    with a workspace of one tile (bitwise equal), against complex128 position by position.
+    Each of the n positions rounds an entry (arithmetic of up to four terms, then storage)
+    by at most 4 units in the last place of the table's largest entries, and the sweep
+    preserves norms, so an amplitude errs by at most n 2^-22 (complex64) or n 2^-50
+    (complex128) of the largest one; small amplitudes have no relative bound of their own."""
+    import torch
+    for s in range(2000):
+        rng = np.random.default_rng(s)
+        n = {9: 22, 10: 24, 11: 26, 12: 30}[rank]
+        g = pkg.instances.degree_at_most3(n, rng)
+        order = rng.permutation(n).tolist()
+        e = pkg.edges_from_graph(g)
+        if max(pkg.rank_profile(n, e, order)) == rank:
+            break
+    u = pkg.instances.haar_su2(n, rng)
+    plan, single = pkg.ScanPlan(n, e, order), pkg.ScanPlan(n, e, order, fuse=False)
+    bits = pkg.instances.uniform_bits(count, n, rng)
+    rv, rl = pkg.ScanEngine(single, u, precision="c128").sweep_bits(bits)
+    ref = rv * np.exp(rl - 0.35 * n)
+    eng = pkg.ScanEngine(plan, u, precision=precision)
+    v, l = eng.sweep_bits(bits)
+    assert 2 < eng.launch_count(count) < pkg.ScanEngine(single, u, precision=precision).launch_count(count)
+    bound = n * 2.0 ** (-50 if precision == "c128" else -22) * np.abs(ref).max()
+    assert np.abs(v * np.exp(l - 0.35 * n) - ref).max() <= bound
+    small = pkg.ScanEngine(plan, u, precision=precision, batch_tile=16)
+    w, m = small.sweep_bits(bits)
+    assert np.array_equal(v, w) and np.array_equal(l, m)
+    up = lambda x: (x + 255) // 256 * 256  # noqa: E731
+    need = 2 * up((16 << rank) * small.esize) + up(n * 16 * 32) + up(n * 16) + up(n * 16 * 8)
+    small._ws = torch.empty(need, dtype=torch.uint8, device=small.device)
+    small.workspace_bytes = lambda tile: need
+    w, m = small.sweep_bits(bits)
+    assert np.array_equal(v, w) and np.array_equal(l, m)
+
+
 def test_remainder_tile(pkg):
     """A batch's last strings run in the smallest tile that holds them: same results, and the
     launches that the launch count says."""
