@@ -409,19 +409,27 @@ u128 apply_row(const std::vector<u128>& cols, u128 x) {
 // of the positions before it, for levels 0 .. D.size() - 1 of the run from position j.
 // False when a level outgrows kBlockEnds.
 bool close_over(const Plan& p, int j, std::vector<Subspace>& D, int level, u128 v) {
-  std::vector<std::pair<int, u128>> todo{{level, v}};
-  while (!todo.empty()) {
-    const auto [l, x] = todo.back();
-    todo.pop_back();
+  // Every added vector leaves at most two more to add: never more than the vectors that the
+  // levels hold, plus one.
+  struct {
+    u128 x;
+    int l;
+  } todo[(kBlockLen + 1) * Subspace::kMax + 2];
+  int top = 0;
+  todo[top++] = {v, level};
+  while (top) {
+    --top;
+    const u128 x = todo[top].x;
+    const int l = todo[top].l;
     if (!D[l].add(x)) {
       if (D[l].full) return false;
       continue;
     }
     if (D[l].dim() > kBlockEnds) return false;
-    if (l + 1 < (int)D.size()) todo.push_back({l + 1, apply_row(p.steps[j + l].mcols, x)});
+    if (l + 1 < (int)D.size()) todo[top++] = {apply_row(p.steps[j + l].mcols, x), l + 1};
     if (l > 0) {
       const PlanStep& st = p.steps[j + l - 1];
-      todo.push_back({l - 1, apply_row(st.lcols, x) & (one_at(st.r_in) - 1)});
+      todo[top++] = {apply_row(st.lcols, x) & (one_at(st.r_in) - 1), l - 1};
     }
   }
   return true;
@@ -449,17 +457,10 @@ bool make_block(const Plan& p, int j, int k, const std::vector<Subspace>& D, Dev
                 std::vector<unsigned long long>* words_out) {
   if (k < 2 || k > kBlockLen || j < 1 || j + k > p.n) return false;
   auto cmask = [&](int i) { return one_at(p.steps[j + i].r_in) - 1; };
-  DevBlock d{};
-  d.j = j;
-  d.k = k;
-  d.r_in = p.steps[j].r_in;
-  d.r_out = p.steps[j + k - 1].r_out;
-  d.din = D[0].dim();
-  d.dout = D[k].dim();
   // Stages, from the right: a growing position joins the next one unless its pair offset
   // lies in the next one's kernel (or the two are the whole run: the pair kernel's case).
   auto growing = [&](int i) { return p.dev[j + i].mode == MODE_PAIR && p.dev[j + i].ncombos == 1; };
-  std::vector<int> stage_of(k + 1, -1);  // 1: a fused stage starts here, 0: a single one
+  int stage_of[kBlockLen + 1] = {-1, -1, -1, -1, -1, -1, -1};  // 1: a fused stage starts here, 0: a single one
   for (int i = k - 1; i >= 0; --i) {
     bool join = k > 2 && i > 0 && growing(i - 1);
     if (join) {
@@ -470,14 +471,22 @@ bool make_block(const Plan& p, int j, int k, const std::vector<Subspace>& D, Dev
     if (join) --i;
     stage_of[i] = join ? 1 : 0;
   }
-  d.dmax = 0;
+  int dmax = 0;
   for (int i = 0; i <= k; ++i) {
     if (D[i].dim() > kBlockEnds) return false;
-    if (i > 0 && i < k && stage_of[i] >= 0) d.dmax = std::max(d.dmax, D[i].dim());
+    if (i > 0 && i < k && stage_of[i] >= 0) dmax = std::max(dmax, D[i].dim());
   }
-  if (d.dmax > kBlockDim) return false;
-  d.lg = d.r_out - d.dout;
+  if (dmax > kBlockDim) return false;
   if (!words_out) return true;  // feasible; the tables are built for chosen runs only
+  DevBlock d{};
+  d.j = j;
+  d.k = k;
+  d.r_in = p.steps[j].r_in;
+  d.r_out = p.steps[j + k - 1].r_out;
+  d.din = D[0].dim();
+  d.dout = D[k].dim();
+  d.dmax = dmax;
+  d.lg = d.r_out - d.dout;
   std::vector<unsigned long long>& words = *words_out;
   auto parity = [](u128 x) {
     return (__builtin_popcountll((uint64_t)x) + __builtin_popcountll((uint64_t)(x >> 64))) & 1;
@@ -661,12 +670,14 @@ void choose_runs(Plan& p, int lo, int hi, double launch, std::vector<DevBlock>& 
                  std::vector<int>& run_len) {
   std::vector<double> best(p.n + 1, 0.0);
   std::vector<int> take(p.n + 1, 1);
+  DevBlock d;
   for (int j = hi - 1; j >= lo; --j) {
     best[j] = HUGE_VAL;
-    std::vector<Subspace> D(1);
+    std::vector<Subspace> D;
+    D.reserve(kBlockLen + 1);
+    D.emplace_back();
     bool open = true;  // a longer run needs larger subspaces at every level
     for (int k = 1; k <= kBlockLen && j + k <= hi; ++k) {
-      DevBlock d;
       open = open && extend_run(p, j, k - 1, D);
       if (k > 1 && (!open || !make_block(p, j, k, D, d, nullptr))) {
         if (!open) break;
@@ -684,7 +695,6 @@ void choose_runs(Plan& p, int lo, int hi, double launch, std::vector<DevBlock>& 
     run_len[j] = take[j];
     // Two positions that the pair kernel covers run there (its rows stay in registers).
     if (take[j] < 2 || (take[j] == 2 && p.pair_at[j] >= 0)) continue;
-    DevBlock d;
     std::vector<Subspace> D(1);
     bool ok = true;
     for (int i = 0; i < take[j]; ++i) ok = ok && extend_run(p, j, i, D);
