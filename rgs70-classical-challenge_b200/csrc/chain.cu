@@ -310,8 +310,8 @@ __global__ void chain_zero_kernel(double* x, long long first, int count) {
 template <typename S, int VE, int CPL, int MODE, int NC>
 cudaError_t launch_gram(dim3 grid, cudaStream_t s, const void* Ein, const DevStep& st, const u64* T, double* partial,
                         int lbt, int unit) {
-  return launch_chained(chain_gram_kernel<S, VE, MODE, NC, CPL>, grid, dim3(256), 0, s, (const S*)Ein, st, T, partial, lbt,
-                        unit);
+  return launch_chained(chained_table(2 * sizeof(S), st.r_in + lbt, 1), chain_gram_kernel<S, VE, MODE, NC, CPL>, grid,
+                        dim3(256), 0, s, (const S*)Ein, st, T, partial, lbt, unit);
 }
 
 // Positions that need the Gram pass: pair mode with two or four combos, merge mode.
@@ -455,7 +455,7 @@ int chain_run(Plan& plan, const double* U, long long count, int mode_given, u64 
                                          j == 0);
         if (e != cudaSuccess) return e;
       }
-      return launch_chained(chain_decide_kernel, dim3((unsigned)Bt), dim3(kDecideThreads), 0, stream, partial,
+      return launch_chained(true, chain_decide_kernel, dim3((unsigned)Bt), dim3(kDecideThreads), 0, stream, partial,
                             L.mass_blocks, analytic, Bt, cnt, j, st.v, U2, mode_given, bits, first, uniforms, plan.n, seed,
                             W + (size_t)j * Bt, out_logp, out_cond1, status);
     };

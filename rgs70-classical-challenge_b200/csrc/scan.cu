@@ -317,8 +317,8 @@ template <typename S, typename M, int VE, int CPL, int MODE, int NC, int NG0>
 cudaError_t launch_row(dim3 grid, cudaStream_t s, const void* Ein, void* Eout, const DevStep& st, const u64* T,
                        const double4* W, const unsigned char* F, const u64* mp, u64* mc, int lbt, int unit,
                        u64 es) {
-  return launch_chained(scan_row_kernel<S, M, VE, MODE, NC, CPL, NG0>, grid, dim3(256), 0, s, (const S*)Ein, (S*)Eout, st,
-                        T, W, F, mp, mc, lbt, unit, es);
+  return launch_chained(chained_table(2 * sizeof(S), st.r_in + lbt, grid.y), scan_row_kernel<S, M, VE, MODE, NC, CPL, NG0>,
+                        grid, dim3(256), 0, s, (const S*)Ein, (S*)Eout, st, T, W, F, mp, mc, lbt, unit, es);
 }
 
 template <typename S, typename M, int VE, int CPL>

@@ -10,8 +10,9 @@ cudaError_t launch_pair_one(dim3 grid, cudaStream_t s, const void* Ein, void* Eo
                             const u64* tables, const double4* WA, const double4* WB, const u64* mp, u64* mA,
                             u64* mc, int lbt, u64 es, double* partial) {
   const size_t smem = GRAM ? (size_t)8 * (1u << lbt) * 4 * sizeof(double) : 0;
-  return launch_chained(scan_pair_kernel<S, M, VE, CA, CB, I, GRAM>, grid, dim3(256), smem, s, (const S*)Ein, (S*)Eout,
-                        P, tables, WA, WB, mp, mA, mc, lbt, es, partial);
+  return launch_chained(chained_table(2 * sizeof(S), P.m + lbt, grid.y), scan_pair_kernel<S, M, VE, CA, CB, I, GRAM>,
+                        grid, dim3(256), smem, s, (const S*)Ein, (S*)Eout, P, tables, WA, WB, mp, mA, mc, lbt, es,
+                        partial);
 }
 
 template <typename S, typename M, int VE, int CA, typename I, bool GRAM>
