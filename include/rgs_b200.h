@@ -130,7 +130,12 @@ int rgs_order_search(int32_t n, int32_t n_edges, const int32_t* edges, const int
  * bitstrings executed together in one interleaved table.  That size lets the sweep run
  * chunks of 8192 bitstrings (several tiles) with one launch per low-rank position for the
  * whole chunk; a smaller workspace (down to two tables of one tile) halves the chunk or,
- * at the least, runs tile by tile, with the same results bit for bit. */
+ * at the least, runs tile by tile, with the same results bit for bit.
+ *
+ * Fused plans take one of three routes by plan, precision and batch: rank <= 12, up to 32 or
+ * from 128 strings: on chip, one launch per call; rank 9 to 12, no fixed vertices, large
+ * batches: runs over all positions; else the streamed sweep of single positions, pairs and
+ * (rank >= 18) runs.  Routes agree to rounding. */
 int rgs_scan_workspace_bytes(const rgs_plan* plan, int32_t batch_tile, int32_t precision, size_t* bytes);
 /* Largest batch_tile accepted for a precision (128 complex64, 256 complex64/float32 math,
  * 64 complex128). */
@@ -161,7 +166,8 @@ int rgs_scan_contract(rgs_plan* plan, const double* fvec, int64_t batch, int32_t
  * conditional p(x_v | prefix) from one read of the table (both branches), and the
  * chosen branch is then one scan step.  Extends the reference's p(x) path
  * (W/upstream_scan/gpu_kernel.py:125-170) to sampling and conditional marginals;
- * plans with fixed vertices are not supported.  batch_tile <= 128 (64 for C128).
+ * plans with fixed vertices are not supported.  Fused plans of rank <= 12 with batch_tile
+ * >= 64 run on chip, one launch per call.  batch_tile <= 128 (64 for C128).
  * Workspace: rgs_chain_workspace_bytes().  check != 0 synchronises and reports a branch
  * pair of zero total mass as RGS_ERR_ZERO_NORM. */
 int rgs_chain_workspace_bytes(const rgs_plan* plan, int32_t batch_tile, int32_t precision, size_t* bytes);
@@ -194,7 +200,7 @@ int rgs_chain_marginals(rgs_plan* plan, const double* unitaries, const uint64_t*
  * over ScanOracle.amplitude / the scan sweep (W/scan_oracle.py:19-28,
  * W/upstream_scan/gpu_kernel.py:125-170) for instances of rank <= rgs_batch_max_rank()
  * (13 for complex64, 12 for complex128).  Amplitudes are bitwise equal to
- * rgs_scan_amplitudes; samples use the Philox uniforms of rgs_chain_sample (same seed,
+ * rgs_scan_amplitudes of a plan without fusion; samples use the Philox uniforms of rgs_chain_sample (same seed,
  * same item -> same uniforms).  Plans with fixed vertices: amplitudes only.
  * Every buffer of a batch lives on one device; a plan must outlive the batches that
  * use it.  Adding instances is synchronous (it uploads the plan's tables once per
