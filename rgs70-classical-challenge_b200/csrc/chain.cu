@@ -57,7 +57,7 @@ constexpr int kDecideThreads = 128;  // threads of the per-item decision block
 //   M_x / s^2 = G00 |U_x0|^2 + G11 |U_x1|^2 + 2 Re(G01 U_x0 conj(U_x1)),
 // one accumulation for the two branches.  Layout and geometry as scan_row_kernel.
 template <typename S, int VE, int MODE, int NC, int CPL>
-__global__ void __launch_bounds__(256, 2) chain_gram_kernel(const S* __restrict__ Ein, const __grid_constant__ DevStep st,
+__global__ void __launch_bounds__(256, 2) chain_gram_kernel(const S* Ein, const __grid_constant__ DevStep st,
                                                             const u64* __restrict__ T, double* __restrict__ partial,
                                                             int lbt, int unit_input) {
   constexpr int U = RowsPerIter<NC, CPL, LoadsInFlight<S, double>::value>::value;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256, 2) chain_gram_kernel(const S* __restrict_
 // x_v drawn with the item's uniform (x = 0 iff u (M0 + M1) < M0) or taken from the given
 // bits; then the chosen branch's weights for the step kernel, the sampled bit,
 // log p(x_v | prefix) and the conditional probability p(x_v = 1 | prefix).
-__global__ void chain_decide_kernel(const double* __restrict__ partial, int nblocks, int analytic, int Bt, int count,
+__global__ void chain_decide_kernel(const double* partial, int nblocks, int analytic, int Bt, int count,
                                     int j, int v, const double2* __restrict__ U, int mode_given, u64* __restrict__ bits,
                                     long long first, const double* __restrict__ uniforms, int n, u64 seed,
                                     double4* __restrict__ Wj, double* __restrict__ logp, float* __restrict__ cond1,

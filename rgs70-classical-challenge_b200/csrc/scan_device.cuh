@@ -20,12 +20,13 @@
 #define RGS_PAIR_LOADS 8
 #endif
 // RGS_STREAM_HINTS: table rows are read once and written once per pass, so loads and
-// stores may carry the evict-first (streaming) cache hint.
+// stores may carry the evict-first (streaming) cache hint.  Loads are ordinary (coherent)
+// ones: the row, pair and Gram kernels may start early (chained_start below).
 #ifdef RGS_STREAM_HINTS
 #define RGS_LD(p) __ldcs(p)
 #define RGS_ST(p, v) __stcs(p, v)
 #else
-#define RGS_LD(p) __ldg(p)
+#define RGS_LD(p) (*(p))
 #define RGS_ST(p, v) (*(p) = (v))
 #endif
 
@@ -36,7 +37,15 @@ typedef unsigned long long u64;
 // Start of a kernel that launch_chained starts before its predecessor in the stream has
 // finished: lets its own successor start as early, then waits until the predecessor's
 // grid has completed and its writes are visible.  Nothing before this call may touch
-// global memory.  Without the launch attribute both are no-ops.
+// global memory.  The wait returns at once in a kernel launched without the attribute; the
+// release takes effect whenever the successor has it.
+//
+// The wait makes the predecessor's writes visible to ordinary loads only.  Up to three
+// kernels of a chain are resident together, so what an earlier one of them writes (tables,
+// weights, maxima, Gram partials) is written within this kernel's lifetime and must not go
+// through the read-only path (__ldg, or const __restrict__, which lets the compiler choose
+// it): that path may return what the memory held before.  Only plan data and the caller's
+// inputs, complete before the first kernel of the chain starts, are read that way.
 __device__ __forceinline__ void chained_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

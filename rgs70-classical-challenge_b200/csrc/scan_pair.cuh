@@ -83,9 +83,9 @@ struct PairBlocks {
 // Bt x 4 doubles).  B's weights are not read.
 template <typename S, typename M, int VE, int CA, int CB, typename I, bool GRAM = false>
 __global__ void __launch_bounds__(256, PairBlocks<S, M>::value)
-    scan_pair_kernel(const S* __restrict__ Ein, S* __restrict__ Eout, const __grid_constant__ DevPair P,
-                     const u64* __restrict__ tables, const double4* __restrict__ WA, const double4* __restrict__ WB,
-                     const u64* __restrict__ maxprev, u64* __restrict__ maxA, u64* __restrict__ maxcur, int lbt,
+    scan_pair_kernel(const S* Ein, S* __restrict__ Eout, const __grid_constant__ DevPair P,
+                     const u64* __restrict__ tables, const double4* WA, const double4* WB,
+                     const u64* maxprev, u64* __restrict__ maxA, u64* __restrict__ maxcur, int lbt,
                      u64 e_stride, double* __restrict__ partial) {
   using MA = PairMode<CA>;
   using MB = PairMode<CB>;

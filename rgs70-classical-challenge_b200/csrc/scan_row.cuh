@@ -49,11 +49,11 @@ struct ChunkGroup {
 };
 
 template <typename S, typename M, int VE, int MODE, int NC, int CPL, int NG0>
-__global__ void __launch_bounds__(256, 2) scan_row_kernel(const S* __restrict__ Ein, S* __restrict__ Eout,
+__global__ void __launch_bounds__(256, 2) scan_row_kernel(const S* Ein, S* __restrict__ Eout,
                                                        const __grid_constant__ DevStep st,
-                                                       const u64* __restrict__ T, const double4* __restrict__ W,
-                                                       const unsigned char* __restrict__ F,
-                                                       const u64* __restrict__ maxprev, u64* __restrict__ maxcur,
+                                                       const u64* __restrict__ T, const double4* W,
+                                                       const unsigned char* F,
+                                                       const u64* maxprev, u64* __restrict__ maxcur,
                                                        int lbt, int unit_input, u64 e_stride) {
   constexpr int CPLG = ChunkGroup<S, M, CPL>::value;
   constexpr int U = RowsPerIter<NC, CPLG, LoadsInFlight<S, M>::value>::value;
