@@ -53,11 +53,12 @@ __device__ __forceinline__ void chained_start() {
 
 // Launch with programmatic stream serialisation: the blocks are placed while the previous
 // kernel of the stream drains, which hides the launch latency of short dependent kernels
-// (a chain-rule tile is some 180 of them, 3 us each of which one is the gap).  Only for
-// kernels that begin with chained_start(), and only while their table is short
-// (chained_table): a long kernel has nothing to hide, and its blocks, placed on SMs as they
-// drain instead of evenly on an empty GPU, run longer (rank 30, samples by the chain rule:
-// 33.7 a second against 34.2 without).
+// (a chain-rule tile of 128 strings at n = 40, rank 20 is 85 launches of 17.6 us on average:
+// 512 samples 6.44 -> 5.99 ms).  Only for kernels that begin with chained_start(), and only
+// while the table they work on is short (chained_table): a long kernel has nothing to hide,
+// and its blocks, placed on SMs as they drain instead of evenly on an empty GPU, run longer
+// (rank 30, samples by the chain rule: 33.7 a second against 34.2 without).  The decision
+// kernel has no table and a few short blocks; it starts early everywhere (chain.cu).
 constexpr u64 kChainedBytes = 1ull << 26;
 inline bool chained_table(int entry, int log_entries, unsigned tiles) {
   return ((u64)entry * tiles << log_entries) <= kChainedBytes;
