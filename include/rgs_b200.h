@@ -80,8 +80,8 @@ int rgs_plan_step_tables(const rgs_plan* plan, int32_t j, uint64_t* tables, int3
  * vertices as one pass (scan_pair_kernel) that keeps the table between them out of
  * memory, choosing non-overlapping pairs that keep the most entries out of HBM.
  * rgs_plan_set_fusion(plan, 0) turns this off, (…, 1) back on; only before the plan's
- * first use on a device (RGS_ERR_ARG after).  Amplitudes agree to rounding either way;
- * a (value, logscale) pair of the two schedules may differ by an exact power of two. */
+ * first use on a device (RGS_ERR_ARG after).  (value, logscale) has the same bits either
+ * way (short of underflow within a table; the log-scale of a zero value may differ). */
 int rgs_plan_set_fusion(rgs_plan* plan, int32_t on);
 /* Number of fused pairs and (if first_positions is not NULL) position j of each,
  * int32[count]. */
@@ -135,7 +135,8 @@ int rgs_order_search(int32_t n, int32_t n_edges, const int32_t* edges, const int
  * Fused plans take one of three routes by plan, precision and batch: rank <= 12, up to 32 or
  * from 128 strings: on chip, one launch per call; rank 9 to 12, no fixed vertices, large
  * batches: runs over all positions; else the streamed sweep of single positions, pairs and
- * (rank >= 18) runs.  Routes agree to rounding. */
+ * (rank >= 18) runs.  A string's (value, logscale) has the same bits on every route, so it does
+ * not depend on the batch, the tile or the workspace. */
 int rgs_scan_workspace_bytes(const rgs_plan* plan, int32_t batch_tile, int32_t precision, size_t* bytes);
 /* Largest batch_tile accepted for a precision (128 complex64, 256 complex64/float32 math,
  * 64 complex128). */
@@ -200,7 +201,7 @@ int rgs_chain_marginals(rgs_plan* plan, const double* unitaries, const uint64_t*
  * over ScanOracle.amplitude / the scan sweep (W/scan_oracle.py:19-28,
  * W/upstream_scan/gpu_kernel.py:125-170) for instances of rank <= rgs_batch_max_rank()
  * (13 for complex64, 12 for complex128).  Amplitudes are bitwise equal to
- * rgs_scan_amplitudes of a plan without fusion; samples use the Philox uniforms of rgs_chain_sample (same seed,
+ * rgs_scan_amplitudes; samples use the Philox uniforms of rgs_chain_sample (same seed,
  * same item -> same uniforms).  Plans with fixed vertices: amplitudes only.
  * Every buffer of a batch lives on one device; a plan must outlive the batches that
  * use it.  Adding instances is synchronous (it uploads the plan's tables once per

@@ -290,6 +290,11 @@ bool make_pair(Plan& p, int j, DevPair& out, std::vector<unsigned long long>& mb
   }
   d.dw = dw;
   for (int k = 0; k < 3; ++k) d.piv[k] = k < dw ? piv[k] : 0;
+  if (cB == PC_P2F || cB == PC_P4H || cB == PC_M2) {
+    const int own = highest_bit(basisB[0]);
+    if (std::find(piv.begin(), piv.end(), own) == piv.end()) return false;  // cannot happen: W contains basisB[0]
+    d.swapB = pairA && bit_of(tA, own) ? 1 : 0;
+  }
   d.tabA_off = dA.table_off;
   d.nbA = dA.nbytes;
   std::vector<u128> tab;
@@ -309,7 +314,9 @@ bool make_pair(Plan& p, int j, DevPair& out, std::vector<unsigned long long>& mb
   return true;
 }
 
-// Chooses the fused pairs: non-overlapping (j, j + 1) with j >= 1, inside one of the
+// Chooses the fused pairs: non-overlapping (j, j + 1) with j >= 1 and j + 1 < n - 1 (the last
+// position runs alone, scaled from the true maximum of the table before it: the exponents
+// then sum to that maximum's own, whatever the passes before), inside one of the
 // leading / middle / trailing runs, maximising the intermediate entries kept out of
 // HBM (2^m each); rebuilds p.pairs and p.pair_at.
 void build_pairs(Plan& p) {
@@ -328,7 +335,7 @@ void build_pairs(Plan& p) {
   std::vector<DevPair> cand(p.n);
   std::vector<char> ok(p.n, 0);
   std::vector<unsigned long long> scratch;
-  for (int j = 1; j + 1 < p.n; ++j) {
+  for (int j = 1; j + 2 < p.n; ++j) {
     if (region(j) != region(j + 1)) continue;
     scratch.clear();
     ok[j] = make_pair(p, j, cand[j], scratch) ? 1 : 0;
@@ -595,6 +602,12 @@ bool make_block(const Plan& p, int j, int k, const std::vector<Subspace>& D, Dev
     d.pair[sg] = pair ? (int)place(tloc) : 0;
     d.twin[sg] = fused ? (int)place(vloc) : 0;
     d.twin_sign[sg] = fused ? parity(sa.ycol & sb.beta) : 0;
+    if (fused) {
+      const u128 off = (sa.ycol ^ apply_cols(sb.lcols, apply_cols(sb.mcols, sa.ycol))) & cmask(ib);
+      while (d.twin_order[sg] < db.ncombos && (((u128)db.combos[d.twin_order[sg]] ^ off) & cmask(ib))) ++d.twin_order[sg];
+      // Cannot happen: off lies in the kernel, and has y bit 0 like L_B M_B t_A and t_A.
+      if (d.twin_order[sg] >= (pair ? db.ng0 : db.ncombos)) return false;
+    }
     for (unsigned c = 0; c < (1u << D[o].dim()); ++c) {
       if ((pair && ((c >> pt) & 1)) || (fused && ((c >> pv) & 1))) continue;
       const u128 l0 = apply_cols(sb.lcols, D[o].at(c));
@@ -711,7 +724,8 @@ void choose_runs(Plan& p, int lo, int hi, double launch, std::vector<DevBlock>& 
 }
 
 // Runs of the middle positions of large plans (rank >= kBlockRank), and of every position
-// of plans whose tables are just small enough for chunks of tiles (kFlatRank and above).
+// but the last (see build_pairs) of plans whose tables are just small enough for chunks of
+// tiles (kFlatRank and above).
 void build_blocks(Plan& p) {
   p.blocks.clear();
   p.block_at.assign(p.n, -1);
@@ -726,8 +740,8 @@ void build_blocks(Plan& p) {
   small_runs(p, h, t);
   if (p.rmax >= kBlockRank && std::max(h, 1) < t)
     choose_runs(p, std::max(h, 1), t, 4096.0, p.blocks, p.block_at, p.run_len);
-  if (p.rmax >= kFlatRank && p.rmax <= kSmallRank && p.n > 1)
-    choose_runs(p, 1, p.n, 256.0, p.flat_blocks, p.flat_at, p.flat_len);
+  if (p.rmax >= kFlatRank && p.rmax <= kSmallRank && p.n > 2)
+    choose_runs(p, 1, p.n - 1, 256.0, p.flat_blocks, p.flat_at, p.flat_len);
 }
 
 // On-chip step records (plans of rank <= kResMaxRank): see ResStep.

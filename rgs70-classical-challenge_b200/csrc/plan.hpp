@@ -114,6 +114,11 @@ struct DevPair {
   int piv[3];                    // pivot bits of W (ascending): a group's q0 has zeros there
   int codeA, codeB;              // PairCode of A and B
   int j;                         // position A
+  // Order of B's terms.  The unfused step sums over L_B c' ^ combos, where L_B c' has no bit
+  // of B's kappa-0 kernel vector's own column (its highest bit).  q0 has none either (that
+  // bit is a pivot of W); q0 ^ t_A has it where t_A does, and then the rows i ^ 2 of odd i
+  // change places.
+  int swapB;
 };
 
 // A run of k consecutive free positions j .. j + k - 1 as one pass (scan_block_kernel): the
@@ -151,6 +156,9 @@ struct DevBlock {
   int pair[kBlockLen];            // offset of a pair's second output (slot or local row)
   int twin[kBlockLen];            // fused: offset of the outputs of the partner gathers
   int twin_sign[kBlockLen];       // fused: parity(t_A & beta_B)
+  // Fused: the twin of combo c's row is row c ^ twin_order of the twin operation's own sum
+  // (L_B M_B t_A = t_A ^ combo[twin_order]; see DevPair::swapB).
+  int twin_order[kBlockLen];
   unsigned merges;                // bit i: position j + i is a merge (weights f(0) +- f(1))
   int words;                      // program words
   unsigned long long tab_off;     // u64 index: per (byte, value) the pair (x_0 | x_k << 32,
@@ -188,7 +196,7 @@ struct Plan {
   // fused pair), 0 where no segment starts or outside the middle positions.
   std::vector<DevBlock> blocks;
   std::vector<int> block_at, run_len;
-  // The same over every position but the first (kFlatRank <= rank <= kSmallRank).
+  // The same over every position but the first and the last (kFlatRank <= rank <= kSmallRank).
   std::vector<DevBlock> flat_blocks;
   std::vector<int> flat_at, flat_len;
   bool exec_ok = false;

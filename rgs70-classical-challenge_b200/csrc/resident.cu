@@ -200,14 +200,18 @@ __device__ __forceinline__ void one_row(unsigned qu, const unsigned (&cm)[NC], c
       const unsigned sgn = (((qu ^ cm[c]) << 16) & 0x80000000u) ^ w.ovs;
       const M er = (M)e[c].x, ei = (M)e[c].y;
       if (PAIR) {
-        const M nr = flip31(er, sgn), ni = flip31(ei, sgn);
-        if (c < NG0) {
+        // wA terms first in both outputs (scan_row.cuh).
+        if (c < NG0)
           cmad(oa, er, ei, wA);
-          cmad(ob, nr, ni, wB);
-        } else {
-          cmad(oa, nr, ni, wB);
-          cmad(ob, er, ei, wA);
-        }
+        else
+          cmad(oa, flip31(er, sgn), flip31(ei, sgn), wB);
+        const int d = (c + NG0) % NC;
+        const unsigned sgd = (((qu ^ cm[d]) << 16) & 0x80000000u) ^ w.ovs;
+        const M dr = (M)e[d].x, di = (M)e[d].y;
+        if (d < NG0)
+          cmad(ob, flip31(dr, sgd), flip31(di, sgd), wB);
+        else
+          cmad(ob, dr, di, wA);
       } else {
         cmad(oa, er, ei, sgn ? wB : wA);
       }

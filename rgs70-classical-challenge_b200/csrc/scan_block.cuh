@@ -8,7 +8,11 @@
 // one contiguous piece of a row.
 //
 // Arithmetic per entry as in the position-by-position sweep: same combos in the same
-// order, every interior entry rounded to the storage type.  Renormalisation as in the
+// order, every interior entry rounded to the storage type, also where a fused stage keeps
+// it in registers, so that a string's result has the bits of the position-by-position sweep
+// (complex64 with float64 arithmetic: 4096 strings at n = 40 18.7 ms without that rounding,
+// 21.0 with it; one order of sums for all schedules cost 1% in float32 arithmetic, 2% at
+// rank 11).  Renormalisation as in the
 // pair kernel: the first position is scaled from the previous maximum, the others by the
 // power of two of their own weights (2^0 for a row of a unitary), recorded as the maximum
 // 4^e / 4 of the interior tables so that the finalisation's exponents add up.
@@ -82,6 +86,8 @@ struct BlockLane {
     *reinterpret_cast<V*>(p) = v;
     mx[0] = fmax(mx[0], norm2(v.x, v.y));
   }
+  // As if the entry had been stored between two positions.
+  static __device__ __forceinline__ void store_rounded(E& e) { e.re = (M)(S)e.re, e.im = (M)(S)e.im; }
   static __device__ __forceinline__ R zero() { return (M)0; }
   static __device__ __forceinline__ R mad(R a, R b, R c) { return fma(a, b, c); }
   static __device__ __forceinline__ R neg(R a) { return -a; }
@@ -122,6 +128,7 @@ struct BlockLane<float, float, 2> {
     mx[0] = fmaxf(mx[0], norm2(e.re.x, e.im.x));
     mx[1] = fmaxf(mx[1], norm2(e.re.y, e.im.y));
   }
+  static __device__ __forceinline__ void store_rounded(E&) {}
   static __device__ __forceinline__ R zero() { return make_float2(0.f, 0.f); }
   static __device__ __forceinline__ R mad(R a, R b, R c) { return f2fma(a, b, c); }
   static __device__ __forceinline__ R neg(R a) { return make_float2(-a.x, -a.y); }
@@ -168,7 +175,9 @@ struct BlockStep {
 // B: combo c's gathered entry e gives the two rows e f_A(0) and +-e f_A(1) of A's output;
 // the one with the gather's y bit goes to the operation itself, the other to its twin
 // (same kappa pattern, own signs), so both of A's outputs are used as they are formed.
-template <typename L, typename S, int NV, bool FUSED, bool PAIR, int NC, int NG0, bool FIRST, bool LAST, int U>
+// TW: DevBlock::twin_order as a constant; swapping the registers at run time is slower where
+// the peak runs decide (16384 strings at n = 40: 46.1 ms constant, 46.6 swapped).
+template <typename L, typename S, int NV, bool FUSED, bool PAIR, int NC, int NG0, bool FIRST, bool LAST, int TW, int U>
 __device__ __forceinline__ void block_ops(const BlockOp* __restrict__ ops, const BlockStep& g,
                                           const BlockCoef<typename L::R>& wa, const BlockCoef<typename L::R>& wb,
                                           const BlockCoef<typename L::R>& pa, const BlockCoef<typename L::R>& pb,
@@ -191,39 +200,57 @@ __device__ __forceinline__ void block_ops(const BlockOp* __restrict__ ops, const
   }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    E a[NT], b[NT];
+    E a[NT], b[NT], x[NC][NT];
+    unsigned m[NC][NT];  // bit 31: the term's sign
 #pragma unroll
     for (int t = 0; t < NT; ++t) a[t] = b[t] = E{L::zero(), L::zero()};
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-      E x[NT];
-      x[0] = e[u][c];
+      m[c][0] = sign[u] << c;
+      x[c][0] = e[u][c];
       if constexpr (FUSED) {
+        m[c][NT - 1] = m[c][0] ^ g.twin_sign;
         E p{L::zero(), L::zero()}, q{L::zero(), L::zero()};
         block_mad<L>(p, e[u][c].re, e[u][c].im, pa);
         block_mad<L>(q, L::flip(e[u][c].re, sign[u] << (4 + c)), L::flip(e[u][c].im, sign[u] << (4 + c)), pb);
+        L::store_rounded(p);
+        L::store_rounded(q);
         const bool y = (sign[u] << (8 + c)) & 0x80000000u;
-        x[0].re = y ? q.re : p.re;
-        x[0].im = y ? q.im : p.im;
-        x[NT - 1].re = y ? p.re : q.re;
-        x[NT - 1].im = y ? p.im : q.im;
+        x[c][0].re = y ? q.re : p.re;
+        x[c][0].im = y ? q.im : p.im;
+        x[c][NT - 1].re = y ? p.re : q.re;
+        x[c][NT - 1].im = y ? p.im : q.im;
       }
+    }
+    // wa terms first in both outputs of a pair (scan_row.cuh): a over the rows in order, b
+    // from row NG0 on, then the rows before it; the twin's rows in its own order.
+    auto add_b = [&](int c) {
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        const unsigned m = (sign[u] << c) ^ (t ? g.twin_sign : 0u);
-        if (PAIR) {
-          const typename L::R nr = L::flip(x[t].re, m), ni = L::flip(x[t].im, m);
-          if (c < NG0) {
-            block_mad<L>(a[t], x[t].re, x[t].im, wa);
-            block_mad<L>(b[t], nr, ni, wb);
-          } else {
-            block_mad<L>(a[t], nr, ni, wb);
-            block_mad<L>(b[t], x[t].re, x[t].im, wa);
-          }
-        } else {
-          block_mad<L>(a[t], x[t].re, x[t].im, (m & 0x80000000u) ? wb : wa);
-        }
+        const int q = t ? c ^ TW : c;
+        if (c < NG0)
+          block_mad<L>(b[t], L::flip(x[q][t].re, m[q][t]), L::flip(x[q][t].im, m[q][t]), wb);
+        else
+          block_mad<L>(b[t], x[q][t].re, x[q][t].im, wa);
       }
+    };
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const int q = t ? c ^ TW : c;
+        if (!PAIR)
+          block_mad<L>(a[t], x[q][t].re, x[q][t].im, (m[q][t] & 0x80000000u) ? wb : wa);
+        else if (c < NG0)
+          block_mad<L>(a[t], x[q][t].re, x[q][t].im, wa);
+        else
+          block_mad<L>(a[t], L::flip(x[q][t].re, m[q][t]), L::flip(x[q][t].im, m[q][t]), wb);
+      }
+      if (PAIR && (NG0 == NC || c >= NG0)) add_b(c);
+    }
+    if constexpr (PAIR && NG0 < NC) {
+#pragma unroll
+      for (int c = 0; c < NG0; ++c) add_b(c);
     }
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
@@ -241,7 +268,7 @@ __device__ __forceinline__ void block_ops(const BlockOp* __restrict__ ops, const
 }
 
 // A stage's row operations (a power of two), U at a time or, below U, one by one.
-template <typename L, typename S, int NV, bool FUSED, bool PAIR, int NC, int NG0, bool FIRST, bool LAST>
+template <typename L, typename S, int NV, bool FUSED, bool PAIR, int NC, int NG0, bool FIRST, bool LAST, int TW>
 __device__ __forceinline__ void block_rows(const BlockOp* __restrict__ ops, int rows, const BlockStep& g,
                                            const BlockWeights<L>& w, const BlockWeights<L>& wp, S (&mx)[NV]) {
   constexpr int LOADS = FUSED ? 4 : 8;
@@ -251,26 +278,39 @@ __device__ __forceinline__ void block_rows(const BlockOp* __restrict__ ops, int 
   if (U > 1 && rows < U) {
 #pragma unroll 1
     for (int r = 0; r < rows; ++r)
-      block_ops<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, 1>(ops + r, g, wa, wb, pa, pb, mx);
+      block_ops<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, TW, 1>(ops + r, g, wa, wb, pa, pb, mx);
     return;
   }
 #pragma unroll 1
   for (int r = 0; r < rows; r += U)
-    block_ops<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, U>(ops + r, g, wa, wb, pa, pb, mx);
+    block_ops<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, TW, U>(ops + r, g, wa, wb, pa, pb, mx);
 }
 
 template <typename L, typename S, int NV, bool FUSED, bool FIRST, bool LAST>
-__device__ __forceinline__ void block_stage(int code, const BlockOp* ops, int rows, const BlockStep& g,
+__device__ __forceinline__ void block_stage(int code, int twin_order, const BlockOp* ops, int rows, const BlockStep& g,
                                             const BlockWeights<L>& w, const BlockWeights<L>& wp, S (&mx)[NV]) {
-#define RGS_BLOCK_ROWS(PAIR, NC, NG0) block_rows<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST>(ops, rows, g, w, wp, mx)
-  switch (code) {
-    case RC_P1: RGS_BLOCK_ROWS(true, 1, 1); break;
-    case RC_P2H: RGS_BLOCK_ROWS(true, 2, 1); break;
-    case RC_P2F: RGS_BLOCK_ROWS(true, 2, 2); break;
-    case RC_P4H: RGS_BLOCK_ROWS(true, 4, 2); break;
-    case RC_P4F: RGS_BLOCK_ROWS(true, 4, 4); break;
-    case RC_M1: RGS_BLOCK_ROWS(false, 1, 1); break;
-    default: RGS_BLOCK_ROWS(false, 2, 2); break;
+#define RGS_BLOCK_ROWS(PAIR, NC, NG0, TW) \
+  block_rows<L, S, NV, FUSED, PAIR, NC, NG0, FIRST, LAST, FUSED ? TW : 0>(ops, rows, g, w, wp, mx)
+  switch (FUSED ? code | twin_order << 3 : code) {
+    case RC_P1: RGS_BLOCK_ROWS(true, 1, 1, 0); break;
+    case RC_P2H: RGS_BLOCK_ROWS(true, 2, 1, 0); break;
+    case RC_P2F: RGS_BLOCK_ROWS(true, 2, 2, 0); break;
+    case RC_P4H: RGS_BLOCK_ROWS(true, 4, 2, 0); break;
+    case RC_P4F: RGS_BLOCK_ROWS(true, 4, 4, 0); break;
+    case RC_M1: RGS_BLOCK_ROWS(false, 1, 1, 0); break;
+    case RC_M2: RGS_BLOCK_ROWS(false, 2, 2, 0); break;
+    default:
+      if constexpr (FUSED) {
+        switch (code | twin_order << 3) {
+          case RC_P2F | 1 << 3: RGS_BLOCK_ROWS(true, 2, 2, 1); break;
+          case RC_P4H | 1 << 3: RGS_BLOCK_ROWS(true, 4, 2, 1); break;
+          case RC_P4F | 1 << 3: RGS_BLOCK_ROWS(true, 4, 4, 1); break;
+          case RC_P4F | 2 << 3: RGS_BLOCK_ROWS(true, 4, 4, 2); break;
+          case RC_P4F | 3 << 3: RGS_BLOCK_ROWS(true, 4, 4, 3); break;
+          case RC_M2 | 1 << 3: RGS_BLOCK_ROWS(false, 2, 2, 1); break;
+          default: break;  // make_block gives no other
+        }
+      }
   }
 #undef RGS_BLOCK_ROWS
 }
@@ -400,17 +440,17 @@ __global__ void __launch_bounds__(kBlockThreads, MINB)
         g.twin_sign = (unsigned)P.twin_sign[i] << 31;
         const BlockWeights<L> wp = wts[pos * T + tid];
         if (i == 0)
-          block_stage<L, S, NV, true, true, false>(P.code[i], op, P.rows[i], g, w, wp, mx);
+          block_stage<L, S, NV, true, true, false>(P.code[i], P.twin_order[i], op, P.rows[i], g, w, wp, mx);
         else if (last)
-          block_stage<L, S, NV, true, false, true>(P.code[i], op, P.rows[i], g, w, wp, mx);
+          block_stage<L, S, NV, true, false, true>(P.code[i], P.twin_order[i], op, P.rows[i], g, w, wp, mx);
         else
-          block_stage<L, S, NV, true, false, false>(P.code[i], op, P.rows[i], g, w, wp, mx);
+          block_stage<L, S, NV, true, false, false>(P.code[i], P.twin_order[i], op, P.rows[i], g, w, wp, mx);
       } else if (i == 0) {
-        block_stage<L, S, NV, false, true, false>(P.code[i], op, P.rows[i], g, w, w, mx);
+        block_stage<L, S, NV, false, true, false>(P.code[i], 0, op, P.rows[i], g, w, w, mx);
       } else if (last) {
-        block_stage<L, S, NV, false, false, true>(P.code[i], op, P.rows[i], g, w, w, mx);
+        block_stage<L, S, NV, false, false, true>(P.code[i], 0, op, P.rows[i], g, w, w, mx);
       } else {
-        block_stage<L, S, NV, false, false, false>(P.code[i], op, P.rows[i], g, w, w, mx);
+        block_stage<L, S, NV, false, false, false>(P.code[i], 0, op, P.rows[i], g, w, w, mx);
       }
     }
   }

@@ -13,8 +13,8 @@
 // unscaled (the scale of an intermediate table is not known until the whole table
 // exists) and the pass records max |E|^2 = 1/4 for A, whose exponent is 0, so the
 // finalisation's sum of exponents stays exact; B's maximum is recorded as usual and
-// scales the position after B.  A value therefore differs from the unfused sweep's by an
-// exact power of two in (value, logscale), not in the amplitude value * 2^logscale.
+// scales the position after B.  The tables differ from the unfused sweep's by exact powers
+// of two; as the last position is never fused, (value, logscale) has the same bits.
 //
 // Lanes: a lane owns one 16-byte chunk column of every row it touches (VE items);
 // rows of more than 32 chunks are split into 32-chunk column slices, one slice per
@@ -153,6 +153,10 @@ __global__ void __launch_bounds__(256, PairBlocks<S, M>::value)
   }
   __syncthreads();
 
+  // Parities of the intermediate rows in the order that B sums them (DevPair::swapB).
+  constexpr bool kSwap = MA::pair && !GRAM && (CB == PC_P2F || CB == PC_P4H || CB == PC_M2);
+  const unsigned pwB = kSwap && P.swapB ? (P.pwB & 0x55u) | ((P.pwB & 0x22u) << 2) | ((P.pwB & 0x88u) >> 2) : P.pwB;
+
   const u64* T2 = tables + P.tab2_off;
   const I maskA = (I)P.maskA, betaA = (I)P.betaA, betaB = (I)P.betaB;
   const u64 groups = 1ull << (P.m - P.dw);
@@ -222,14 +226,16 @@ __global__ void __launch_bounds__(256, PairBlocks<S, M>::value)
 #pragma unroll
             for (int k = 0; k < NCA; ++k) {
               const M er = (M)e[u][a][k].re(v), ei = (M)e[u][a][k].im(v);
-              const M nr = flip_sign(er, pa[u][a][k]), ni = flip_sign(ei, pa[u][a][k]);
-              if (k < MA::ng0) {
+              if (k < MA::ng0)
                 cmad(x, er, ei, wAa[v]);
-                cmad(y, nr, ni, wAb[v]);
-              } else {
-                cmad(x, nr, ni, wAb[v]);
-                cmad(y, er, ei, wAa[v]);
-              }
+              else
+                cmad(x, flip_sign(er, pa[u][a][k]), flip_sign(ei, pa[u][a][k]), wAb[v]);
+              const int q = (k + MA::ng0) % NCA;  // wA terms first (scan_row.cuh)
+              const M qr = (M)e[u][a][q].re(v), qi = (M)e[u][a][q].im(v);
+              if (q < MA::ng0)
+                cmad(y, flip_sign(qr, pa[u][a][q]), flip_sign(qi, pa[u][a][q]), wAb[v]);
+              else
+                cmad(y, qr, qi, wAa[v]);
             }
             const S xr = (S)x.re, xi = (S)x.im, yr = (S)y.re, yi = (S)y.im;
             const bool sw = ya[u][a];
@@ -282,24 +288,37 @@ __global__ void __launch_bounds__(256, PairBlocks<S, M>::value)
           }
           continue;
         }
-        // B: the group's output rows from the registers.
+        if constexpr (kSwap) {
+          if (P.swapB) {
+#pragma unroll
+            for (int i = 1; i < NW; i += 4) {
+              const S tr = ir[i], ti = ii[i];
+              ir[i] = ir[i + 2], ii[i] = ii[i + 2];
+              ir[i + 2] = tr, ii[i + 2] = ti;
+            }
+          }
+        }
+        // B: the group's output rows from the registers, wA terms first (scan_row.cuh).
 #pragma unroll
         for (int b = 0; b < NUB; ++b) {
           Cx<M> x{(M)0, (M)0}, y{(M)0, (M)0};
 #pragma unroll
           for (int a = 0; a < NCB; ++a) {
             const int i = MA::pair ? (a << 1) | b : a;
-            const int par = pq[u] ^ (int)((P.pwB >> i) & 1u);
+            const int par = pq[u] ^ (int)((pwB >> i) & 1u);
             const M er = (M)ir[i], ei = (M)ii[i];
             if (MB::pair) {
-              const M nr = flip_sign(er, par), ni = flip_sign(ei, par);
-              if (a < MB::ng0) {
+              if (a < MB::ng0)
                 cmad(x, er, ei, wBa[v]);
-                cmad(y, nr, ni, wBb[v]);
-              } else {
-                cmad(x, nr, ni, wBb[v]);
-                cmad(y, er, ei, wBa[v]);
-              }
+              else
+                cmad(x, flip_sign(er, par), flip_sign(ei, par), wBb[v]);
+              const int q = (a + MB::ng0) % NCB, iq = MA::pair ? (q << 1) | b : q;
+              const int parq = pq[u] ^ (int)((pwB >> iq) & 1u);
+              const M qr = (M)ir[iq], qi = (M)ii[iq];
+              if (q < MB::ng0)
+                cmad(y, flip_sign(qr, parq), flip_sign(qi, parq), wBb[v]);
+              else
+                cmad(y, qr, qi, wBa[v]);
             } else {
               cmad(x, er, ei, par ? wBb[v] : wBa[v]);
             }

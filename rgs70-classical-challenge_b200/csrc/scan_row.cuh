@@ -20,10 +20,16 @@
 // PAIR without per-item selects.  The y bit of gather k is y_k = y(p0) ^ kappa_k, where
 // kappa_k is bit r_in of combo k, a constant of the step; the compiler orders the combos
 // with kappa = 0 first (NG0 of them).  With X = sum_{k<NG0} e wA + sum_{k>=NG0} (-1)^par e wB
-// and Y = sum_{k<NG0} (-1)^par e wB + sum_{k>=NG0} e wA, row c' receives X and row c'^t
+// and Y = sum_{k>=NG0} e wA + sum_{k<NG0} (-1)^par e wB, row c' receives X and row c'^t
 // receives Y when y(p0) = 0, and the other way round when y(p0) = 1: the choice is one
 // swap of the two store addresses per row, and the sign is applied to the gathered value
 // (exactly the negated product), so no weight is selected per item.
+//
+// Order of the sums: the wA terms first, in X and in Y, so that the rounding of a row does
+// not depend on which of the pair stands for it: L t is e_y (same gathers, X and Y swapped)
+// or, where the y column depends on the others, e_y ^ vec_y (gathers shifted by vec_y, the
+// first with y bit 1).  Every schedule (single positions, fused pairs, runs, on chip) thus
+// computes the same bits up to its power-of-two scales.
 #pragma once
 #include "scan_device.cuh"
 
@@ -186,15 +192,19 @@ __global__ void __launch_bounds__(256, 2) scan_row_kernel(const S* Ein, S* __res
             for (int k = 0; k < NC; ++k) {
               const int par = pc[u][k] ^ ov[i];
               if (MODE == MODE_PAIR) {
+                // Both outputs sum their wA terms first (X: gathers 0 .., Y: NG0 ..).
                 const M pr = (M)e[u][k][jj].re(v), pi = (M)e[u][k][jj].im(v);
-                const M nr = flip_sign(pr, par), ni = flip_sign(pi, par);
-                if (k < NG0) {
+                if (k < NG0)
                   cmad(oa, pr, pi, wA[i]);
-                  cmad(ob, nr, ni, wB[i]);
-                } else {
-                  cmad(oa, nr, ni, wB[i]);
-                  cmad(ob, pr, pi, wA[i]);
-                }
+                else
+                  cmad(oa, flip_sign(pr, par), flip_sign(pi, par), wB[i]);
+                constexpr int kFirst = NG0 % NC;
+                const int q = (k + kFirst) % NC, parq = pc[u][q] ^ ov[i];
+                const M qr = (M)e[u][q][jj].re(v), qi = (M)e[u][q][jj].im(v);
+                if (q < NG0)
+                  cmad(ob, flip_sign(qr, parq), flip_sign(qi, parq), wB[i]);
+                else
+                  cmad(ob, qr, qi, wA[i]);
               } else if (MODE == MODE_MERGE) {
                 const M er = (M)e[u][k][jj].re(v), ei = (M)e[u][k][jj].im(v);
                 cmad(oa, er, ei, par ? wB[i] : wA[i]);
