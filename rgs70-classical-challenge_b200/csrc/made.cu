@@ -61,27 +61,51 @@ __device__ __forceinline__ uint4 load8_partial(const __nv_bfloat16* src, int val
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Eight consecutive bf16 values of rows whose chunks are `unit` elements (8, 4, 2 or 1)
+// aligned; those at index >= valid replaced by zero.
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* src, int valid, int unit) {
+  if (valid < 8) return load8_partial(src, valid);
+  if (unit == 1) return load8_partial(src, 8);
+  if (unit == 8) return __ldg(reinterpret_cast<const uint4*>(src));
+  if (unit == 4) {
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(src)), b = __ldg(reinterpret_cast<const uint2*>(src) + 1);
+    return make_uint4(a.x, a.y, b.x, b.y);
+  }
+  const unsigned* p = reinterpret_cast<const unsigned*>(src);
+  return make_uint4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
+// Elements of the widest load that row starts `ld` apart from `p` allow.
+__device__ __forceinline__ int row_unit(const __nv_bfloat16* p, int ld) {
+  const unsigned low = (unsigned)(uintptr_t)p | (unsigned)ld * 2u;
+  return (low & 15u) == 0 ? 8 : ((low & 7u) == 0 ? 4 : ((low & 3u) == 0 ? 2 : 1));
+}
+
 // Rows [r0, r0 + 128) x k [k0, k0 + 64) of a logical R x K operand into the K-major
 // layout; zero outside the operand.  kmajor: element (r, k) at G[r * ld + k]; otherwise
 // at G[k * ld + r] (MN-major: transposed in registers on the way).  128 threads, one
-// 8 x 8 core matrix each; vec: 16-byte loads are aligned (ld % 8 == 0, G 16-byte aligned).
+// 8 x 8 core matrix each; unit: row_unit of the operand.  Loads of
+// two bytes bound the kernel (4096 x 500 x 500: 104 us, with the 8-byte loads that its rows
+// allow 32; 4096 x 501 x 501, whole chunks loaded without a test per element: 118 -> 71).
 __device__ __forceinline__ void stage_tile(unsigned char* tile, const __nv_bfloat16* __restrict__ G, int ld, int R,
-                                           int K, int r0, int k0, bool kmajor, bool vec) {
+                                           int K, int r0, int k0, bool kmajor, int unit) {
   const int t = threadIdx.x;
   if (kmajor) {
     const int kc = t & 7, rg = t >> 3;
     const int k = k0 + kc * 8;
+    uint4 rows[8];  // all loaded before the first is stored
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int ii = (i + kc) & 7;  // rotated so that a quarter warp hits distinct banks
-      const int r = r0 + rg * 8 + ii;
+      const int r = r0 + rg * 8 + ((i + kc) & 7);  // rotated so that a quarter warp hits distinct banks
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < R && k < K) {
         const __nv_bfloat16* src = G + (size_t)r * ld + k;
-        v = (vec && k + 8 <= K) ? __ldg(reinterpret_cast<const uint4*>(src)) : load8_partial(src, K - k);
+        v = load8(src, K - k, unit);
       }
-      *reinterpret_cast<uint4*>(tile + cm_off(rg * 8 + ii, kc)) = v;
+      rows[i] = v;
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(tile + cm_off(rg * 8 + ((i + kc) & 7), kc)) = rows[i];
   } else {
     const int rg = t & 15, kc = t >> 4;
     const int r = r0 + rg * 8;
@@ -92,7 +116,8 @@ __device__ __forceinline__ void stage_tile(unsigned char* tile, const __nv_bfloa
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (k < K && r < R) {
         const __nv_bfloat16* src = G + (size_t)k * ld + r;
-        v = (vec && r + 8 <= R) ? __ldg(reinterpret_cast<const uint4*>(src)) : load8_partial(src, R - r);
+        // Two-byte loads: one path for the whole warp, whose lanes meet the ragged end here.
+        v = unit == 1 ? load8_partial(src, R - r) : load8(src, R - r, unit);
       }
       rows[j] = v;
     }
@@ -177,8 +202,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_c
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const bool vecA = (g.lda % 8 == 0) && (((uintptr_t)g.A & 15) == 0);
-  const bool vecB = (g.ldb % 8 == 0) && (((uintptr_t)g.B & 15) == 0);
+  const int unitA = row_unit(g.A, g.lda), unitB = row_unit(g.B, g.ldb);
   // This block's K slices [k0, k0 + KT).
   const int slices = (g.K + TBK - 1) / TBK;
   const int per = (slices + split - 1) / split, rank = split > 1 ? (int)tc::cluster_rank() : 0;
@@ -227,10 +251,10 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_c
     // are waited for (also bounded) before the block frees its TMEM.
     int consumed = 0;
     if (threadIdx.x == 32) {
-      int issued = 0;
+      int issued = 0, s = 0;
+      uint32_t phase = 1;  // of the stage's last use: kt / kTmaStages - 1
       for (int kt = 0; kt < KT; ++kt) {
-        const int s = kt % kTmaStages;
-        if (kt >= kTmaStages && !tc::mbar_wait(&bars[s], (uint32_t)(kt / kTmaStages - 1) & 1u)) {
+        if (kt >= kTmaStages && !tc::mbar_wait(&bars[s], phase)) {
           ok = false;
           break;
         }
@@ -238,18 +262,38 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_c
         tc::mbar_expect_tx(&full[s], 2 * kTileBytes);
         load(kt, As, As + kTileBytes, &full[s]);
         ++issued;
+        if (++s == kTmaStages) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
       s_issued = issued;
     } else if (threadIdx.x == 0) {
+      // Descriptors by additions to the first stage's (built anew for each MMA, they and the
+      // divisions by the stage count cost 1.5 us of 15.6 at 8192 x 512 x 512).  The address
+      // field holds 16-byte units.
+      const uint32_t first = tc::smem_u32(base);
+      const uint64_t a_first = desc(first, 1, maps.mn_a, 0), b_first = desc(first + kTileBytes, 1, maps.mn_b, 0);
+      const uint32_t a_step = maps.mn_a ? 2048 >> 4 : 32 >> 4, b_step = maps.mn_b ? 2048 >> 4 : 32 >> 4;
+      int s = 0;
+      uint32_t phase = 0;
       for (int kt = 0; kt < KT; ++kt) {
-        const int s = kt % kTmaStages;
-        if (!tc::mbar_wait(&full[s], (uint32_t)(kt / kTmaStages) & 1u)) {
+        if (!tc::mbar_wait(&full[s], phase)) {
           ok = false;
           break;
         }
         ++consumed;
         tc::fence_after_sync();
-        multiply(kt, s);
+        const uint32_t stage = (uint32_t)s * (2 * kTileBytes >> 4);
+#pragma unroll
+        for (int kk = 0; kk < TBK / 16; ++kk)
+          tc::mma_f16(tmem, a_first + (stage + kk * a_step), b_first + (stage + kk * b_step), idesc,
+                      (kt > 0 || kk > 0) ? 1u : 0u);
+        tc::mma_commit(&bars[s]);
+        if (++s == kTmaStages) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
       if (consumed > 0 &&
           !tc::mbar_wait(&bars[(consumed - 1) % kTmaStages], (uint32_t)((consumed - 1) / kTmaStages) & 1u))
@@ -274,8 +318,8 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_c
         load(kt, As, Bs, &full[s]);
       }
       const int k = (k0 + kt) * TBK;
-      if (!maps.tma_a) stage_tile(As, g.A, g.lda, g.M, g.K, m0, k, !g.transA, vecA);
-      if (!maps.tma_b) stage_tile(Bs, g.B, g.ldb, g.N, g.K, n0, k, g.transB != 0, vecB);
+      if (!maps.tma_a) stage_tile(As, g.A, g.lda, g.M, g.K, m0, k, !g.transA, unitA);
+      if (!maps.tma_b) stage_tile(Bs, g.B, g.ldb, g.N, g.K, n0, k, g.transB != 0, unitB);
       tc::fence_async_smem();
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -293,7 +337,10 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_c
   tc::fence_after_sync();
   if (!ok && threadIdx.x == 0) atomicExch(&g_tc_timeout, 1);
   const uint32_t tmem_row = tmem + ((uint32_t)(warp * 32) << 16);
-  const bool aligned = (g.ldc & 7) == 0 && ((uintptr_t)g.C & 15) == 0 && ((uintptr_t)g.Cb & 15) == 0 &&
+  // Rows of whole 16-byte chunks: of the FP32 output (four columns), and of the bf16 output
+  // and gate (eight) where there are such.  (8192 x 500 x 512, FP32 output: 13.6 us, element
+  // by element 44.)
+  const bool aligned = (g.ldc & (g.Cb || g.gate ? 7 : 3)) == 0 && ((uintptr_t)g.C & 15) == 0 && ((uintptr_t)g.Cb & 15) == 0 &&
                        ((uintptr_t)g.gate & 15) == 0 && (!g.mask || ((g.N & 15) == 0 && ((uintptr_t)g.mask & 15) == 0));
   if (split == 1) {
     const int m = m0 + warp * 32 + lane;
@@ -338,6 +385,17 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_c
             for (int q = 0; q < 2; ++q)
               dst[q] = make_uint4(pack_bf16(v[8 * q], v[8 * q + 1]), pack_bf16(v[8 * q + 2], v[8 * q + 3]),
                                   pack_bf16(v[8 * q + 4], v[8 * q + 5]), pack_bf16(v[8 * q + 6], v[8 * q + 7]));
+          }
+          continue;
+        }
+        if (aligned && !g.Cb && !g.mask && !g.gate && (g.N & 3) == 0) {  // the last columns, by fours
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (n + 4 * q >= g.N) break;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = finish(g, __uint_as_float(r[4 * q + j]), m, n + 4 * q + j);
+            *reinterpret_cast<float4*>(g.C + (size_t)m * g.ldc + n + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
           }
           continue;
         }
@@ -605,7 +663,8 @@ int gemm_bf16(const GemmArgs& g, cudaStream_t s) {
     maps.mn_b = maps.tma_b && !g.transB;
   }
   // Split K where a long K meets few tiles (weight gradients: K is the batch): up to eight
-  // blocks per tile, at least four slices each.  Shorter sums (K < 1024) stay in one
+  // blocks per tile, four slices or more each but for the last of a cluster (33 slices over
+  // eight blocks: six of 5, one of 3, one of none).  Shorter sums (K < 1024) stay in one
   // accumulator, in slice order.
   const int tiles = ((g.N + TBN - 1) / TBN) * ((g.M + TBM - 1) / TBM), slices = (g.K + TBK - 1) / TBK;
   int split = 1;
