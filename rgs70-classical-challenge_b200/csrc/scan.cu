@@ -448,11 +448,11 @@ namespace {
 struct Segment {
   int j, len, pair, block;
 };
-std::vector<Segment> segments_of(const Plan& plan, int from, int to, bool flat = false) {
+std::vector<Segment> segments_of(const Plan& plan, int from, int to, bool flat = false, bool runs = true) {
   std::vector<Segment> out;
   for (int j = from; j < to;) {
     // 0: not planned as runs
-    const int run = flat ? plan.flat_len[j] : (plan.blocks.empty() ? 0 : plan.run_len[j]);
+    const int run = flat ? plan.flat_len[j] : (plan.blocks.empty() || !runs ? 0 : plan.run_len[j]);
     const int block = !run ? -1 : (flat ? plan.flat_at[j] : plan.block_at[j]);
     const int pa = plan.pair_at.empty() ? -1 : plan.pair_at[j];
     if (block >= 0) {
@@ -527,6 +527,11 @@ bool scan_flat(const Plan& plan, int precision, long long batch) {
   return r >= 10 && batch >= (r >= 13 ? 512 : 1ll << (23 - r));
 }
 
+bool scan_runs(const Plan& plan, int precision, int Bt) {
+  if (Bt > 1 || precision == RGS_PREC_C128) return true;
+  return plan.rmax < 21 || plan.rmax > (precision == RGS_PREC_C64_F32 ? 25 : 22);
+}
+
 bool scan_on_chip(const Plan& plan, int precision, long long batch) {
   if (!plan.fuse || !resident_plan_fits(plan)) return false;
   if (batch > kOnChipFew && batch < kOnChipMany) return false;
@@ -567,12 +572,14 @@ int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, 
     total = batch ? 1 : 0;
   } else if (S < 2) {
     total = (batch + Bt - 1) / Bt *
-            ((long long)segments_of(plan, 0, (int)n, scan_flat(plan, precision, batch)).size() + 2);
+            ((long long)segments_of(plan, 0, (int)n, scan_flat(plan, precision, batch), scan_runs(plan, precision, Bt))
+                 .size() +
+             2);
   } else {
     const long long stride = (long long)S * Bt;
     const bool flat = scan_flat(plan, precision, batch);
     const long long nh = (long long)segments_of(plan, 0, C.h, flat).size();
-    const long long nm = (long long)segments_of(plan, C.h, C.t).size();
+    const long long nm = (long long)segments_of(plan, C.h, C.t, false, scan_runs(plan, precision, Bt)).size();
     const long long nt = (long long)segments_of(plan, std::max(C.t, C.h), (int)n, flat).size();
     for (long long first = 0; first < batch; first += stride) {
       const long long tiles = (std::min(stride, batch - first) + Bt - 1) / Bt;
@@ -645,7 +652,7 @@ int scan_run_tiles(Plan& plan, const double* U, const u64* bits, const double* f
   const u64* tables = (const u64*)dc->tables;
   long long launches = 0;
   const bool flat = scan_flat(plan, precision, batch);
-  const std::vector<Segment> segs = segments_of(plan, 0, plan.n, flat);
+  const std::vector<Segment> segs = segments_of(plan, 0, plan.n, flat, scan_runs(plan, precision, Bt));
 
   for (long long first = 0; first < batch; first += Bt) {
     const int count = (int)std::min<long long>(Bt, batch - first);
@@ -728,7 +735,7 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
   const int lbt = __builtin_ctz((unsigned)Bt);
   long long launches = 0;
   const bool flat = scan_flat(plan, precision, batch);
-  const std::vector<Segment> head = segments_of(plan, 0, h, flat), mid = segments_of(plan, h, t),
+  const std::vector<Segment> head = segments_of(plan, 0, h, flat), mid = segments_of(plan, h, t, false, scan_runs(plan, precision, Bt)),
                              tail = segments_of(plan, std::max(t, h), n, flat);
 
   for (long long first = 0; first < batch; first += stride) {

@@ -58,6 +58,14 @@ bool scan_on_chip(const Plan& plan, int precision, long long batch);
 // = 26); rank 10, 4096 strings 125 / 155, 8192 197 / 186; complex128, rank 12, 300 strings
 // 194 / 161, 1000 419 / 204; rank 9, 4096 strings 119 / 111 and 87 / 93, 8192 192 / 131.
 bool scan_flat(const Plan& plan, int precision, long long batch);
+// Whether the runs of a plan's middle positions are used on tiles of Bt strings; else its pairs
+// are.  Not for a single string in a window of ranks, where rows of 8 bytes make a run's
+// gathers the slower ones (pairs / runs, two instances per rank): float32 arithmetic, rank 20
+// 165 / 140 and 205 / 170 us, 21 177 / 170 and 224 / 285, 22 198 / 235 and 277 / 419, 24 539 /
+// 604, 25 421 / 476 and 844 / 854, 26 584 / 650 and 936 / 831, 27 1456 / 1129; float64
+// arithmetic, rank 21 189 / 173 and 237 / 270, 22 219 / 216 and 292 / 379, 23 293 / 267 and 383 /
+// 356.  Two strings: rank 22 261 / 245, 24 661 / 536.
+bool scan_runs(const Plan& plan, int precision, int Bt);
 // The passes of a streamed sweep: first position and number of positions of each.
 void scan_segments(const Plan& plan, std::vector<int>& first, std::vector<int>& length);
 // Kernel launches scan_run queues for `batch` items with that workspace.

@@ -28,7 +28,7 @@
 //     has no slots: 16 slots per column instead of 32, and half the column traffic (4096
 //     strings 13.8 -> 11.6 ms, 5000 strings in complex128 25.7 -> 21.0 ms);
 //   * float32 arithmetic carries two strings per thread (packed FMAs, one set of index work
-//     for both).
+//     for both) in launches large enough (launch_block).
 // Fetching the next group's maps ahead changed nothing (11.6 ms), prefetching its rows into
 // L2 cost 4%.
 #pragma once

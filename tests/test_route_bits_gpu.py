@@ -87,7 +87,7 @@ def test_tiles_of_streamed_plans(pkg, precision):
         plan, single = pkg.ScanPlan(n, e, order), pkg.ScanPlan(n, e, order, fuse=False)
         bits = pkg.instances.uniform_bits(70, n, rng)
         ref = pkg.ScanEngine(single, u, precision=precision, batch_tile=8).sweep_bits(bits)
-        for tile in (1, 2, 16, pkg.max_batch_tile(precision)):
+        for tile in (1, 2, 16, 64, pkg.max_batch_tile(precision)):
             eng = pkg.ScanEngine(plan, u, precision=precision, batch_tile=tile)
             assert eng.launch_count(70) > 1
             _same(eng.sweep_bits(bits), ref, (plan.rmax, tile))
@@ -115,3 +115,22 @@ def test_chain_and_batch(pkg, precision):
             k = rb.add(g, u, order, bits)
             rb.run()
             _same(rb.amplitudes(k)[:2], ref, plan.rmax)
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("rank", [21, 23])
+def test_single_strings(pkg, precision, rank):
+    """One string per tile, where complex64 plans of some ranks keep their pairs instead of
+    runs, and remainder tiles of one, against single positions."""
+    rng = np.random.default_rng(rank)
+    for n, e, order, u in _instances(pkg, rank, rank, 1, 60 + rank, (44, 52)):
+        bits = pkg.instances.uniform_bits(5, n, rng)
+        ref = pkg.ScanEngine(pkg.ScanPlan(n, e, order, fuse=False), u, precision=precision, batch_tile=2).sweep_bits(bits)
+        plan = pkg.ScanPlan(n, e, order)
+        counts = {}
+        for tile in (1, 4):
+            eng = pkg.ScanEngine(plan, u, precision=precision, batch_tile=tile)
+            counts[tile] = eng.launch_count(tile)
+            _same(eng.sweep_bits(bits), ref, (rank, tile))
+        pairs = precision == "c64f32" or (precision == "c64" and rank == 21)
+        assert (counts[1] > counts[4]) == pairs
