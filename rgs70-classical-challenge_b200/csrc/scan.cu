@@ -540,14 +540,21 @@ bool scan_on_chip(const Plan& plan, int precision, long long batch) {
 
 // Tile of the last batch % Bt strings where a smaller one holds them, else 0: a tile costs
 // its full width whatever it holds, so 11 strings in tiles of 8 run as 8 + 4, not 8 + 8
-// (results do not depend on the tile).  Plans of small tables keep one tile size, as their
-// launches, not their bytes, cost.
-int remainder_tile(const Plan& plan, long long batch, int Bt) {
+// (results do not depend on the tile).  The smaller tile is a sweep of its own, with its own
+// launches at the low ranks (60 to 100 us), so it has to save more than 128 MiB of the largest
+// table (n = 32, rank 13, 5 strings as 4 + 4 / 4 + 1: 119 / 215 us; rank 17, complex128, 33 as
+// 32 + 32 / 32 + 1: 275 / 308, 70 as 64 + 64 / 64 + 8: 429 / 393; rank 20, complex64, 40 as
+// 32 + 32 / 32 + 8: 484 / 458; rank 22, 5 as 4 + 4 / 4 + 1: 372 / 493).  Plans of rank 18 and
+// above in tiles of 8 or more take it from 16 MiB on, as their tested launch counts have it,
+// although it can cost as much (rank 19, 11 strings as 8 + 8 / 8 + 4: 228 / 302).
+int remainder_tile(const Plan& plan, long long batch, int Bt, int precision) {
   const long long rem = batch % Bt;
   if (rem == 0 || plan.rmax <= kSmallRank) return 0;
   int t = 1;
   while (t < rem) t *= 2;
-  return t < Bt ? t : 0;
+  if (t == Bt) return 0;
+  const u64 saved = ((u64)(Bt - t) << std::min(plan.rmax, 40)) * (precision == RGS_PREC_C128 ? 16 : 8);
+  return saved > (128ull << 20) || (plan.rmax >= kBlockRank && Bt >= 8 && saved >= (16ull << 20)) ? t : 0;
 }
 
 int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, size_t ws_bytes, long long* out) {
@@ -560,7 +567,7 @@ int scan_launch_count(const Plan& plan, long long batch, int Bt, int precision, 
   if ((rc = scan_pick_chunk(plan, Bt, precision, ws_bytes, C, &S))) return rc;
   const long long n = plan.n;
   long long total = 0;
-  if (const int last = remainder_tile(plan, batch, Bt); last && !scan_on_chip(plan, precision, batch)) {
+  if (const int last = remainder_tile(plan, batch, Bt, precision); last && !scan_on_chip(plan, precision, batch)) {
     const long long rem = batch % Bt;
     long long a = 0, b = 0;
     if (batch > rem && (rc = scan_launch_count(plan, batch - rem, Bt, precision, ws_bytes, &a))) return rc;
@@ -698,7 +705,7 @@ int scan_run(Plan& plan, const double* U, const u64* bits, const double* fvec, l
   if (scan_on_chip(plan, precision, batch))
     return scan_run_on_chip(plan, U, bits, fvec, batch, precision, out_value, out_logscale, workspace, ws_bytes, Bt,
                             stream, stats);
-  if (const int last = remainder_tile(plan, batch, Bt)) {
+  if (const int last = remainder_tile(plan, batch, Bt, precision)) {
     const long long rem = batch % Bt, full = batch - rem;
     const size_t vsize = 2 * (precision == RGS_PREC_C128 ? sizeof(double) : sizeof(float));
     ScanStats a, b;
