@@ -515,6 +515,9 @@ bool make_block(const Plan& p, int j, int k, const std::vector<Subspace>& D, Dev
     const PlanStep &sa = p.steps[j + i], &sb = p.steps[j + ib];
     const DevStep& db = p.dev[j + ib];
     const bool pair = db.mode == MODE_PAIR, last = o == k;
+    // One position consumes one bit of the basis, so its kernel has one dimension without the
+    // y column: four combos always include y bits (RC_P4H), and the run kernel has no RC_P4F.
+    if (pair && db.ncombos == 4 && db.ng0 == 4) return false;
     // Input row (level i) of a row of level ib, and A's y bit there.
     auto input_of = [&](u128 row) { return fused ? apply_cols(sa.lcols, row) & cmask(i) : row; };
     unsigned tloc = 0, vloc = 0;

@@ -296,7 +296,6 @@ __device__ __forceinline__ void block_stage(int code, int twin_order, const Bloc
     case RC_P2H: RGS_BLOCK_ROWS(true, 2, 1, 0); break;
     case RC_P2F: RGS_BLOCK_ROWS(true, 2, 2, 0); break;
     case RC_P4H: RGS_BLOCK_ROWS(true, 4, 2, 0); break;
-    case RC_P4F: RGS_BLOCK_ROWS(true, 4, 4, 0); break;
     case RC_M1: RGS_BLOCK_ROWS(false, 1, 1, 0); break;
     case RC_M2: RGS_BLOCK_ROWS(false, 2, 2, 0); break;
     default:
@@ -304,9 +303,6 @@ __device__ __forceinline__ void block_stage(int code, int twin_order, const Bloc
         switch (code | twin_order << 3) {
           case RC_P2F | 1 << 3: RGS_BLOCK_ROWS(true, 2, 2, 1); break;
           case RC_P4H | 1 << 3: RGS_BLOCK_ROWS(true, 4, 2, 1); break;
-          case RC_P4F | 1 << 3: RGS_BLOCK_ROWS(true, 4, 4, 1); break;
-          case RC_P4F | 2 << 3: RGS_BLOCK_ROWS(true, 4, 4, 2); break;
-          case RC_P4F | 3 << 3: RGS_BLOCK_ROWS(true, 4, 4, 3); break;
           case RC_M2 | 1 << 3: RGS_BLOCK_ROWS(false, 2, 2, 1); break;
           default: break;  // make_block gives no other
         }
