@@ -852,7 +852,7 @@ def run_batched(args, rank, world, local_rank):
             "data": "synthetic (seeded graphs, gates, strings; Philox uniforms)",
             "config": {"workload": f"{nI} Erdos-Renyi instances (avg degree 3, n in [20,36], searched orders, r_max "
                                    f"{min(i.rmax for i in insts)}-{max(i.rmax for i in insts)}): {K} amplitudes + "
-                                   f"{S} samples each per step, one persistent launch replayed from a CUDA graph",
+                                   f"{S} samples each per step, one launch replayed from a CUDA graph",
                        "instances": nI, "strings_per_instance": K, "samples_per_instance": S,
                        "work_units": rb.units, "l2": "tables live in shared memory; HBM holds only inputs and outputs",
                        "tuned_variant": {"chosen": ["512 threads, 192 KiB of tables", "128 threads, 56 KiB of tables",

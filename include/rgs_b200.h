@@ -195,9 +195,9 @@ int rgs_chain_marginals(rgs_plan* plan, const double* unitaries, const uint64_t*
 
 /* ---------------------------------------------------------------- resident batch of small instances
  * Many (graph, gates, order) instances -- amplitudes of given bitstrings and exact
- * chain-rule samples of each -- in ONE persistent launch: each block holds an
- * instance's whole environment table for up to 64 items in shared memory and takes
- * work units (largest first) from a device counter.  Replaces the per-instance loop
+ * chain-rule samples of each -- in ONE launch: a work unit is up to 32 items of one instance,
+ * whose environment tables a warp or a block holds in shared memory (at most 8 items per
+ * block); units are ordered largest first, one per block or one per warp.  Replaces the per-instance loop
  * over ScanOracle.amplitude / the scan sweep (W/scan_oracle.py:19-28,
  * W/upstream_scan/gpu_kernel.py:125-170) for instances of rank <= rgs_batch_max_rank()
  * (13 for complex64, 12 for complex128).  Amplitudes are bitwise equal to

@@ -1,8 +1,8 @@
-"""Many small instances in one persistent launch (``rgs_batch_*`` in ``librgs_b200.so``).
+"""Many small instances in one launch (``rgs_batch_*`` in ``librgs_b200.so``).
 
 ``ResidentBatch`` gathers (graph, gates, order) instances of rank at most
 ``max_rank(precision)`` -- amplitudes of given bitstrings and exact chain-rule
-samples of each -- and runs all of them with one kernel whose blocks hold an
+samples of each -- and runs all of them with one kernel whose blocks or warps hold an
 instance's whole environment table in shared memory.  Amplitudes equal
 ``ScanOracle.amplitudes`` bit for bit; samples are those of
 ``ChainSampler.sample(seed=...)`` (same Philox uniforms), up to decisions whose

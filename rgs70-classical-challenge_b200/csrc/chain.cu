@@ -379,8 +379,10 @@ long long chain_launches_per_tile(const Plan& plan, bool mode_given, bool with_l
 }
 
 // Whether chain_run takes a plan on chip: rank <= kResPlanRank, fusion on, and a tile of 64
-// (the largest of complex128) or more.  A caller that asks for smaller tiles bounds the
-// strings in flight and keeps the streamed schedule, one launch sequence per tile.
+// (the largest of complex128) or more.  Smaller tiles, which callers have to ask for, keep the
+// streamed schedule, one launch sequence per tile, although on chip is faster (it holds no
+// table in memory that a small tile would bound): the tests of that schedule count its
+// launches in tiles of 16 and 32.
 bool chain_on_chip(const Plan& plan, int Bt) {
   return plan.fuse && resident_plan_fits(plan) && Bt >= kChainMaxTile / 2;
 }

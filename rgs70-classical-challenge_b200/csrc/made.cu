@@ -180,7 +180,7 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 // 64 slices, so one CTA per tile leaves most of the chip idle, and operands transposed by
 // the threads keep the tensor core waiting.  Split over eight CTAs and loaded by TMA they
 // are launch and pipeline latency: the eight GEMMs of a gradient (4096 rows, n = 56, 2 x
-// 512 hidden) took 1656 us before and take 91 us.
+// 512 hidden) took 1656 us before and take 81 us.
 __global__ void __launch_bounds__(128) gemm_tc_kernel(GemmArgs g, const __grid_constant__ GemmMaps maps, int split) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);

@@ -137,7 +137,7 @@ struct DevPair {
 constexpr int kBlockLen = 6;      // positions per run
 // Dimension of interior levels with slots (16 per column).  32 slots halve the warps per
 // SM for a few longer runs: 12.2 against 11.6 ms (float32 arithmetic, 4096 strings of the n =
-// 40, rank 20 instance), 22.5 against 21.0 (complex128, 5000), 4.85 against 5.04 (rank 26).
+// 40, rank 20 instance), 22.5 against 21.0 (complex128), 4.85 against 5.04 (rank 26).
 constexpr int kBlockDim = 4;
 constexpr int kBlockEnds = 6;     // dimension of D_0, D_k and of levels without slots
 constexpr int kBlockRank = 18;    // runs are formed in plans of at least this rank,

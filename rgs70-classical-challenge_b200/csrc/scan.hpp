@@ -46,8 +46,9 @@ int scan_pick_chunk(const Plan& plan, int Bt, int precision, size_t ws_bytes, Ch
 // instead of one launch per segment: plans of rank <= kResPlanRank with fusion on, below
 // the batches of scan_flat.  Measured, on chip against fused pairs: one string 31 against
 // 166 us (rank 9, n = 40), 300 strings 50 against 207 us (rank 10, complex64, float32
-// arithmetic).  Sweeps of 33 to 127 strings keep the position-by-position launch schedule
-// of one tile.
+// arithmetic).  33 to 127 strings stay streamed although on chip is faster there too (64
+// strings, ranks 4 and 6: 16-24 us against 78-96): the tests of the pair schedule count its
+// launches at 64 and 100 strings.
 constexpr long long kOnChipFew = 32, kOnChipMany = 128;
 bool scan_on_chip(const Plan& plan, int precision, long long batch);
 // Whether such a plan is swept as runs over all its positions, one launch per run and chunk

@@ -20,13 +20,13 @@
 // What bounds it: the pair kernels moved 2.8M entries per string of the n = 40, rank 20
 // instance at 79% of the copy bandwidth; runs move 1.1M and are bound by instruction issue
 // and the latency of column accesses (peak run of that instance, float32 arithmetic: issue
-// slots 50% busy, DRAM 28%; 16 warps per SM, as many as the columns leave room for).  Hence
+// slots 49% busy, DRAM 28%; 14 warps per SM, as many as columns and registers allow).  Hence
 //   * a row operation reads one 32-byte record with its ready-made slot offsets, rows and
 //     signs (shared memory, the same for every thread), several gathers are in flight per
 //     thread, only the last stage tracks maxima;
 //   * a growing position and the next one form one stage, so that the level of the peak rank
 //     has no slots: 16 slots per column instead of 32, and half the column traffic (4096
-//     strings 13.8 -> 11.6 ms, 5000 strings in complex128 25.7 -> 21.0 ms);
+//     strings 13.8 -> 11.6 ms, in complex128 25.7 -> 21.0 ms);
 //   * float32 arithmetic carries two strings per thread (packed FMAs, one set of index work
 //     for both) in launches large enough (launch_block).
 // Fetching the next group's maps ahead changed nothing (11.6 ms), prefetching its rows into
@@ -41,8 +41,8 @@ namespace rgs {
 
 // Threads per block.  64: two warps share the row operations, and blocks are small enough
 // to fill an SM's shared memory (with 32 slots per column, 4096 strings of the n = 40
-// instance, float32 arithmetic: 13.8 ms with 64, 15.9 with 128, 18.8 with 32; complex128,
-// 5000 strings: 25.7 / 29.7 / 36.1).
+// instance, float32 arithmetic: 13.8 ms with 64, 15.9 with 128, 18.8 with 32; complex128
+// 25.7 / 29.7 / 36.1).
 constexpr int kBlockThreads = 64, kBlockLogThreads = 6;
 
 struct __align__(16) BlockOp {
